@@ -17,12 +17,13 @@
 #include <vector>
 
 #include "engine.h"
+#include "grid.cuh"
 #include "share.cuh"
 #include "traverse.cuh"
 
 namespace igxrt {
 
-static_assert(sizeof(BatchItemDev) == 72, "batch item layout");
+static_assert(sizeof(BatchItemDev) == 80, "batch item layout");
 
 struct BatchArgs {
     const BatchItemDev* items;
@@ -81,6 +82,7 @@ template <int LAYOUT, bool MIXED>
 __global__ void __launch_bounds__(256) batch_kernel(BatchArgs a) {
     if (a.times && threadIdx.x == 0)
         atomicMin(a.times, global_ns());
+    constexpr bool GRID = LAYOUT == (int)kLayoutGrid;
     extern __shared__ uint32_t smem[];
     TraversalStack st;
     st.sh = reinterpret_cast<uint2*>(smem) + threadIdx.x;
@@ -153,6 +155,8 @@ __global__ void __launch_bounds__(256) batch_kernel(BatchArgs a) {
                     mode = it->mode;
                     const uint32_t* prev = it->prev;
                     r = load_ray(it->rays, ray, prev ? __ldg(prev + ray) : IGXRT_NO_RAY_HIT);
+                    if (GRID)
+                        to_grid(r, it->grid);
                     best.t = r.tmax_eff;
                     best.u = 0.f;
                     best.v = 0.f;
@@ -190,7 +194,10 @@ __global__ void __launch_bounds__(256) batch_kernel(BatchArgs a) {
             bool occluded = occluded_at_start;
             occluded_at_start = false;
             if (next < 0) {
-                if (MIXED)
+                if (GRID)
+                    occluded = mode ? process_grid_leaf<true, MIXED>(prims, next, r, best)
+                                    : process_grid_leaf<false, MIXED>(prims, next, r, best);
+                else if (MIXED)
                     occluded = mode ? process_leaf_mixed<true>(prims, next, r, best)
                                     : process_leaf_mixed<false>(prims, next, r, best);
                 else
@@ -219,7 +226,9 @@ __global__ void __launch_bounds__(256) batch_kernel(BatchArgs a) {
 using BatchFn = void (*)(BatchArgs);
 
 static BatchFn select_batch_kernel(uint32_t layout, bool mixed) {
-    constexpr int B2 = IGXRT_LAYOUT_BVH2, B4 = IGXRT_LAYOUT_BVH4, B8 = IGXRT_LAYOUT_BVH8;
+    constexpr int B2 = IGXRT_LAYOUT_BVH2, B4 = IGXRT_LAYOUT_BVH4, B8 = IGXRT_LAYOUT_BVH8, G = (int)kLayoutGrid;
+    if (layout == kLayoutGrid)
+        return mixed ? batch_kernel<G, true> : batch_kernel<G, false>;
     if (mixed)
         return layout == B8 ? batch_kernel<B8, true> : layout == B4 ? batch_kernel<B4, true> : batch_kernel<B2, true>;
     return layout == B8 ? batch_kernel<B8, false> : layout == B4 ? batch_kernel<B4, false> : batch_kernel<B2, false>;
@@ -231,9 +240,10 @@ bool aligned(const void* p, size_t a) { return ((uintptr_t)p % a) == 0; }
 
 }  // namespace
 
-void batch_item_for(const igxrt_scene* scene, const igxrt_launch_params& p, const igxrt_ray* rays,
+void batch_item_for(const igxrt_scene* scene, uint32_t layout, const igxrt_ray* rays,
                     const uint32_t* prev, void* out, uint32_t count, uint32_t mode, BatchItemDev& d) {
-    d.nodes = reinterpret_cast<const float4*>(scene->nodes[p.layout]);
+    d.nodes = layout == kLayoutGrid ? scene->grid_nodes : reinterpret_cast<const float4*>(scene->nodes[layout]);
+    d.grid = scene->grid;
     d.prims = reinterpret_cast<const float4*>(scene->prims);
     d.rays = rays;
     d.prev = prev;
@@ -241,7 +251,7 @@ void batch_item_for(const igxrt_scene* scene, const igxrt_launch_params& p, cons
     d.planes = reinterpret_cast<const float4*>(scene->planes);
     d.count = count;
     d.mode = mode;
-    d.node_count = scene->node_count[p.layout];
+    d.node_count = scene->node_count[layout == kLayoutGrid ? IGXRT_LAYOUT_BVH4 : layout];
     d.packet_begin = 0;
     d.plane_count = scene->plane_count;
     d.plane_base = scene->plane_base;
@@ -249,9 +259,14 @@ void batch_item_for(const igxrt_scene* scene, const igxrt_launch_params& p, cons
 
 igxrt_status build_batch_table(igxrt_context* ctx, const igxrt_batch_item* items, uint32_t count,
                                const igxrt_launch_params& p, std::vector<BatchItemDev>& table,
-                               uint32_t& total_packets, uint64_t& total_rays, bool& mixed) {
+                               uint32_t& total_packets, uint64_t& total_rays, bool& mixed,
+                               uint32_t& layout) {
     if (count && !items)
         return fail(ctx, IGXRT_ERROR_INVALID_ARGUMENT, "items is NULL");
+    layout = kLayoutGrid;
+    for (uint32_t i = 0; i < count; ++i)
+        if (items[i].scene && !use_grid(*items[i].scene, p.layout))
+            layout = p.layout;
     table.resize(count);
     uint64_t packets = 0;
     total_rays = 0;
@@ -277,7 +292,7 @@ igxrt_status build_batch_table(igxrt_context* ctx, const igxrt_batch_item* items
             return fail(ctx, IGXRT_ERROR_INVALID_ARGUMENT,
                         format("item %u: batch arrays must be device memory", i));
         BatchItemDev& d = table[i];
-        batch_item_for(it.scene, p, it.rays, it.prev_hit, it.out, it.count, it.mode, d);
+        batch_item_for(it.scene, layout, it.rays, it.prev_hit, it.out, it.count, it.mode, d);
         d.packet_begin = (uint32_t)packets;
         mixed |= it.scene->mixed;
         packets += (it.count + p.packet_size - 1) / p.packet_size;
@@ -291,10 +306,11 @@ igxrt_status build_batch_table(igxrt_context* ctx, const igxrt_batch_item* items
 
 igxrt_status launch_batch(igxrt_context* ctx, const BatchItemDev* d_table, uint32_t count,
                           uint32_t total_packets, uint64_t total_rays, const igxrt_launch_params& p,
-                          uint32_t* queue, cudaStream_t stream, bool mixed, unsigned long long* times) {
+                          uint32_t* queue, cudaStream_t stream, bool mixed, uint32_t layout,
+                          unsigned long long* times) {
     if (total_packets == 0)
         return IGXRT_OK;
-    BatchFn fn = select_batch_kernel(p.layout, mixed);
+    BatchFn fn = select_batch_kernel(layout, mixed);
     const size_t smem = (size_t)p.stack_depth * p.block_size * kStackEntryBytes;
     int per_sm = 0;
     cudaError_t e = allow_smem((const void*)fn, smem);
@@ -385,7 +401,8 @@ igxrt_status igxrt_trace_batch(igxrt_context* ctx, const igxrt_batch_item* items
     uint32_t packets = 0;
     uint64_t rays = 0;
     bool mixed = false;
-    st = build_batch_table(ctx, items, count, p, table, packets, rays, mixed);
+    uint32_t layout = p.layout;
+    st = build_batch_table(ctx, items, count, p, table, packets, rays, mixed, layout);
     if (st != IGXRT_OK || packets == 0)
         return st;
     DeviceGuard guard(ctx->device);
@@ -402,7 +419,7 @@ igxrt_status igxrt_trace_batch(igxrt_context* ctx, const igxrt_batch_item* items
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "batch table upload");
     uint32_t* queue = take_queue_slot(ctx);
-    st = launch_batch(ctx, d_table, count, packets, rays, p, queue, stream, mixed);
+    st = launch_batch(ctx, d_table, count, packets, rays, p, queue, stream, mixed, layout);
     if (st != IGXRT_OK)
         return st;
     // the ring's slots are zero between launches (trace launches skip the
@@ -428,7 +445,8 @@ igxrt_status igxrt_batch_create(igxrt_context* ctx, const igxrt_batch_item* item
     uint32_t packets = 0;
     uint64_t rays = 0;
     bool mixed = false;
-    st = build_batch_table(ctx, items, count, p, table, packets, rays, mixed);
+    uint32_t layout = p.layout;
+    st = build_batch_table(ctx, items, count, p, table, packets, rays, mixed, layout);
     if (st != IGXRT_OK)
         return st;
     DeviceGuard guard(ctx->device);
@@ -456,7 +474,7 @@ igxrt_status igxrt_batch_create(igxrt_context* ctx, const igxrt_batch_item* item
         e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
         st = launch_batch(ctx, static_cast<const BatchItemDev*>(b->d_mem), count, packets, rays, p,
-                          queue, cap, mixed);
+                          queue, cap, mixed, layout);
         cudaGraph_t g = nullptr;
         const cudaError_t e2 = cudaStreamEndCapture(cap, &g);
         b->graph = g;

@@ -81,7 +81,8 @@ igxrt_status resolve_params(igxrt_context* ctx, const igxrt_launch_params& in, i
 
 // One device allocation per scene, 256-byte aligned sub-buffers in this
 // order: BVH2 nodes, BVH4 nodes, records, triangles, planes, parent links of
-// BVH2 and BVH4, refit words, BVH8 nodes, BVH8 slot sources.  Fills every
+// BVH2 and BVH4, refit words, BVH8 nodes, BVH8 slot sources, grid nodes, the
+// grid.  Fills every
 // pointer and count of the scene from `info` and the node counts; the
 // contents are the caller's to write.
 igxrt_status allocate_scene(igxrt_context* ctx, const igxrt_bvh_info& info, uint32_t n2, uint32_t n4,
@@ -104,12 +105,15 @@ igxrt_status allocate_scene(igxrt_context* ctx, const igxrt_bvh_info& info, uint
     const size_t b8 = round_up((size_t)n8 * sizeof(igxrt_bvh8_node), 256);
     const size_t bs8 = round_up((size_t)n8 * 8 * sizeof(uint32_t), 256);
     const size_t o8 = b2 + b4 + bp + bt + bl + bpar + bw;
-    cudaError_t e = cudaMalloc(&s->d_mem, o8 + b8 + bs8);
+    const size_t og = o8 + b8 + bs8, bg = (size_t)n4 * 4 * sizeof(float4);
+    cudaError_t e = cudaMalloc(&s->d_mem, og + bg + 2 * sizeof(float4));
     if (e != cudaSuccess) {
         delete s;
         return cuda_fail(ctx, e, "scene allocation");
     }
     char* base = (char*)s->d_mem;
+    s->grid_nodes = (float4*)(base + og);
+    s->grid = s->grid_nodes + 4 * (size_t)n4;
     s->nodes[IGXRT_LAYOUT_BVH8] = base + o8;
     s->node_count[IGXRT_LAYOUT_BVH8] = n8;
     s->src8 = (const uint32_t*)(base + o8 + b8);
@@ -464,6 +468,15 @@ igxrt_status igxrt_scene_create_from_bvh(igxrt_context* ctx, const igxrt_bvh* bv
     up(s->nodes[IGXRT_LAYOUT_BVH4], bvh->nodes4.data(), bvh->nodes4.size() * sizeof(igxrt_bvh4_node));
     up(s->prims, bvh->prims.data(), bvh->prims.size() * sizeof(igxrt_prim_record));
     up(s->tris, bvh->tris.data(), bvh->tris.size() * sizeof(igxrt_triangle));
+    uint32_t words[kRefitStateWords];
+    if (e == cudaSuccess)
+        e = cudaMemset(s->refit_words, 0, sizeof(words));
+    if (e == cudaSuccess)
+        e = write_grid_nodes(ctx, s, false, nullptr);
+    if (e == cudaSuccess)
+        e = cudaMemcpy(words, s->refit_words, sizeof(words), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess)
+        s->grid_ok = grid_usable(words);
     if (e != cudaSuccess) {
         igxrt_scene_destroy(s);
         return cuda_fail(ctx, e, "scene upload");

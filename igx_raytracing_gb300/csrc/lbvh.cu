@@ -662,11 +662,18 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
     copy(scene->tris, a.obj.tris, sizeof(igxrt_triangle) * (size_t)a.obj.nt);
     copy(scene->planes, a.obj.planes, 16 * (size_t)a.obj.np);
     if (e == cudaSuccess)
+        e = cudaMemsetAsync(scene->refit_words, 0, kRefitStateWords * sizeof(uint32_t), s);
+    if (e == cudaSuccess)
+        e = write_grid_nodes(ctx, scene, false, s);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(w, scene->refit_words, kRefitStateWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
         e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         igxrt_scene_destroy(scene);
         return cuda_fail(ctx, e, "GPU build copy");
     }
+    scene->grid_ok = grid_usable(w);
     *out = scene;
     return IGXRT_OK;
 }

@@ -2,7 +2,7 @@
 //
 // The reference re-uploads its moving spheres every frame and traces them with
 // a linear loop (test/scene/niels_scene.cpp:61-70, res/shaders/trace.glsl:22-46);
-// over a BVH, moved geometry needs the node boxes to follow.  Four passes on
+// over a BVH, moved geometry needs the node boxes to follow.  Five passes on
 // the caller's stream:
 //   1. scan: bounds of every object, max |coordinate| (which sets the padding)
 //      and the scene box, reduced per block, then one atomicMax per block and
@@ -22,7 +22,8 @@
 //      node's slots and its children's unions), and nothing waits on another
 //      thread: a thread either continues or exits;
 //   4. BVH8: every compressed node re-quantized from the BVH2 boxes its slots
-//      were built from (eight lanes per node).
+//      were built from (eight lanes per node);
+//   5. grid nodes: the boxes re-quantized from the BVH4 nodes (grid.cu).
 // Boxes follow the host builder exactly (same min/max argument order, padded by
 // max(2^-18 * max|coordinate|, 1e-30)), so the GPU refit equals igxrt_bvh_refit
 // bit for bit.
@@ -132,7 +133,7 @@ struct RefitArgs {
     float4* unions;  // per node of BVH2, then of BVH4: {lo, 0}, {hi, 0}
 };
 
-static_assert(kRefitStateWords == 8, "refit state words");
+static_assert(kRefitStateWords >= 8, "the scan's words");
 
 // Pass 1: maxabs, scene box and the non-finite check.
 __global__ void __launch_bounds__(kScanBlock) refit_scan_kernel(RefitArgs a) {
@@ -442,7 +443,7 @@ igxrt_status igxrt_scene_refit(igxrt_context* ctx, igxrt_scene* scene, const igx
         refit_nodes_kernel<<<(nodes + 127) / 128, 128, 0, s>>>(a);
     if (a.n8)
         refit_bvh8_kernel<<<(uint32_t)((8 * (uint64_t)a.n8 + 127) / 128), 128, 0, s>>>(a);
-    e = cudaGetLastError();
+    e = write_grid_nodes(ctx, scene, true, s);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "refit launch");
     uint32_t w[kRefitStateWords];
@@ -453,6 +454,7 @@ igxrt_status igxrt_scene_refit(igxrt_context* ctx, igxrt_scene* scene, const igx
         return cuda_fail(ctx, e, "refit");
     if (w[kWordBad])
         return fail(ctx, IGXRT_ERROR_INVALID_ARGUMENT, non_finite_message(w[kWordBad], n));
+    scene->grid_ok = grid_usable(w);
     float maxabs;
     memcpy(&maxabs, &w[kWordMaxAbs], 4);
     scene->info.pad_abs = std::max(maxabs * 0x1p-18f, 1e-30f);

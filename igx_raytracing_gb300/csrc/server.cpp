@@ -185,6 +185,7 @@ bool igxrt_server::launch_one() {
     uint64_t rays = 0;
     uint32_t packets = 0;
     bool mixed = false;
+    uint32_t layout = kLayoutGrid;  // unless a scene of the batch goes without
     // every request in the ready queue, in order, adds its next slice
     for (auto it = ready.begin(); it != ready.end() && s->slices.size() < opt.max_batch_requests;) {
         Request* q = *it;
@@ -200,7 +201,17 @@ bool igxrt_server::launch_one() {
         igxrt_ray* d_rays = reinterpret_cast<igxrt_ray*>(base) + first;
         uint32_t* d_prev = q->r.prev_hit ? reinterpret_cast<uint32_t*>(base + rb) + first : nullptr;
         BatchItemDev& d = s->h_table[s->slices.size()];
-        batch_item_for(sc, params, d_rays, d_prev, base + rb + pb + (size_t)first * elem, n, q->r.mode, d);
+        if (!use_grid(*sc, params.layout) && layout == kLayoutGrid) {
+            layout = params.layout;
+            for (size_t k = 0; k < s->slices.size(); ++k) {
+                const igxrt_scene* other = scenes[s->slices[k].q->r.scene_id];
+                BatchItemDev& o = s->h_table[k];
+                const uint32_t begin = o.packet_begin;
+                batch_item_for(other, layout, o.rays, o.prev, o.out, o.count, o.mode, o);
+                o.packet_begin = begin;
+            }
+        }
+        batch_item_for(sc, layout, d_rays, d_prev, base + rb + pb + (size_t)first * elem, n, q->r.mode, d);
         d.packet_begin = packets;
         packets += (n + params.packet_size - 1) / params.packet_size;
         rays += n;
@@ -221,7 +232,7 @@ bool igxrt_server::launch_one() {
     cudaMemcpyAsync(s->d_table, s->h_table, n * sizeof(BatchItemDev), cudaMemcpyHostToDevice, s->stream);
     cudaMemsetAsync(s->d_times, 0xff, sizeof(unsigned long long), s->stream);
     cudaMemsetAsync(s->d_times + 1, 0, sizeof(unsigned long long), s->stream);
-    igxrt_status st = launch_batch(ctx, s->d_table, n, packets, rays, params, s->queue, s->stream, mixed,
+    igxrt_status st = launch_batch(ctx, s->d_table, n, packets, rays, params, s->queue, s->stream, mixed, layout,
                                    s->d_times);
     const double t = now();
     for (const Slice& sl : s->slices) {

@@ -18,6 +18,7 @@
 
 #include <cstdint>
 
+#include "engine.h"
 #include "igxrt.h"
 #include "internal.h"
 
@@ -192,6 +193,29 @@ struct TraversalStack {
 // Bytes of shared memory per stack entry and thread.
 constexpr uint32_t kStackEntryBytes = 8;
 
+// One triangle record against the ray.  Returns true when an any-hit query is
+// decided (ANY), or when the record became the best hit (closest).
+template <bool ANY>
+__device__ __forceinline__ bool test_record(const float4& v0, const float4& v1, const float4& v2,
+                                            const RayState& r, BestHit& best) {
+    float t, u, v;
+    if (!tri_test(r, v0, v1, v2, t, u, v))
+        return false;
+    const uint32_t prim = __float_as_uint(v0.w);
+    if (t <= r.tmin || prim == r.prev)
+        return false;
+    if (ANY)
+        return t < r.tmax_eff;
+    if (!(t < best.t || (t == best.t && prim < best.prim)))
+        return false;
+    best.t = t;
+    best.u = u;
+    best.v = v;
+    best.prim = prim;
+    best.tcull = cull_limit(t);
+    return true;
+}
+
 // Closest-hit / any-hit leaf processing.  Returns true when an any-hit query
 // is decided (occluder found).
 template <bool ANY, bool COUNT>
@@ -203,22 +227,8 @@ __device__ __forceinline__ bool process_leaf(const float4* __restrict__ prims, i
         const float4 v0 = __ldg(p), v1 = __ldg(p + 1), v2 = __ldg(p + 2);
         if (COUNT)
             ++pf;
-        float t, u, v;
-        if (tri_test(r, v0, v1, v2, t, u, v)) {
-            const uint32_t prim = __float_as_uint(v0.w);
-            if (!(t <= r.tmin) && prim != r.prev) {
-                if (ANY) {
-                    if (t < r.tmax_eff)
-                        return true;
-                } else if (t < best.t || (t == best.t && prim < best.prim)) {
-                    best.t = t;
-                    best.u = u;
-                    best.v = v;
-                    best.prim = prim;
-                    best.tcull = cull_limit(t);
-                }
-            }
-        }
+        if (test_record<ANY>(v0, v1, v2, r, best) && ANY)
+            return true;
         if (__float_as_uint(v1.w))
             break;
         ++i;
@@ -230,6 +240,10 @@ template <int LAYOUT, bool COUNT, bool MIXED>
 __device__ __forceinline__ int32_t visit_node(const float4* __restrict__ nodes, int32_t node,
                                               const RayState& r, const BestHit& best,
                                               TraversalStack& st, bool& overflow, uint32_t& nf);
+
+template <bool MIXED>
+__device__ __forceinline__ int32_t visit_grid(const float4* __restrict__ nodes, int32_t node, const RayState& r,
+                                              float tcull, TraversalStack& st, bool& overflow);
 
 // The node phase of the persistent kernels, called by all 32 lanes of the
 // warp together (every ballot names the whole warp); the lanes with
@@ -255,8 +269,12 @@ __device__ __forceinline__ void node_phase(const float4* __restrict__ nodes, boo
             break;
         if ((uint32_t)__popc(dm) * phase_break <= (uint32_t)__popc(wmask & ~dm))
             break;
-        if (down)
-            next = visit_node<LAYOUT, COUNT, MIXED>(nodes, next, r, best, st, overflow, nf);
+        if (down) {
+            if constexpr (LAYOUT == (int)kLayoutGrid)
+                next = visit_grid<MIXED>(nodes, next, r, best.tcull, st, overflow);
+            else
+                next = visit_node<LAYOUT, COUNT, MIXED>(nodes, next, r, best, st, overflow, nf);
+        }
     }
 }
 
@@ -626,9 +644,61 @@ __device__ __forceinline__ void plane_uv(const RayState& r, const float4& pl, fl
     v = dot3f(ox, oy, oz, zx, zy, zz);
 }
 
-// Leaf of a mixed scene.  Returns true when an any-hit query is decided.
+// Record `i` of a mixed scene against the ray.  Returns true when an any-hit
+// query is decided (ANY), or when the record became the best hit (closest).
 // best_rec (optional): the record index of the best hit so far, for callers
 // that need the hit object's record afterwards (the G-buffer's normals).
+template <bool ANY>
+__device__ __forceinline__ bool test_record_mixed(const float4& v0, const float4& v1, const float4& v2,
+                                                  uint32_t i, const RayState& r, BestHit& best,
+                                                  uint32_t* best_rec = nullptr) {
+    const uint32_t type = __float_as_uint(v2.w), id = __float_as_uint(v0.w);
+    if (id == r.prev)
+        return false;
+    if (type == kPrimTriangle) {
+        float t, u, v;
+        if (!tri_test(r, v0, v1, v2, t, u, v) || t <= r.tmin)
+            return false;
+        if (ANY)
+            return t < r.tmax_eff;
+        if (!better(t, prio_other(id), best))
+            return false;
+        best.t = t;
+        best.u = u;
+        best.v = v;
+        best.prim = prio_other(id);
+    } else if (type == kPrimSphere) {
+        float t;
+        if (!sphere_hit(r, v0.x, v0.y, v0.z, v1.x, t) || !(t >= r.tmin))
+            return false;
+        if (ANY)
+            return t < r.tmax_eff;
+        if (!better(t, prio_other(id), best))
+            return false;
+        sphere_uv(r, v0.x, v0.y, v0.z, t, best.u, best.v);
+        best.t = t;
+        best.prim = prio_other(id);
+    } else {
+        float t, u, v;
+        if (!cube_hit(r, v0, v1, t, u, v))
+            return false;
+        if (ANY)
+            return t < r.tmax_eff;
+        if (!better(t, prio_cube(id), best))
+            return false;
+        best.t = t;
+        best.u = u;
+        best.v = v;
+        best.prim = prio_cube(id);
+    }
+    best.tcull = cull_limit(best.t);
+    if (best_rec)
+        *best_rec = i;
+    return true;
+}
+
+
+// Leaf of a mixed scene.  Returns true when an any-hit query is decided.
 template <bool ANY, bool COUNT = false>
 __device__ __forceinline__ bool process_leaf_mixed(const float4* __restrict__ prims, int32_t ref,
                                                    const RayState& r, BestHit& best, uint32_t* pf = nullptr,
@@ -639,57 +709,8 @@ __device__ __forceinline__ bool process_leaf_mixed(const float4* __restrict__ pr
         const float4 v0 = __ldg(p), v1 = __ldg(p + 1), v2 = __ldg(p + 2);
         if (COUNT)
             ++*pf;
-        const uint32_t type = __float_as_uint(v2.w), id = __float_as_uint(v0.w);
-        if (id != r.prev) {
-            if (type == kPrimTriangle) {
-                float t, u, v;
-                if (tri_test(r, v0, v1, v2, t, u, v) && !(t <= r.tmin)) {
-                    if (ANY) {
-                        if (t < r.tmax_eff)
-                            return true;
-                    } else if (better(t, prio_other(id), best)) {
-                        best.t = t;
-                        best.u = u;
-                        best.v = v;
-                        best.prim = prio_other(id);
-                        best.tcull = cull_limit(t);
-                        if (best_rec)
-                            *best_rec = i;
-                    }
-                }
-            } else if (type == kPrimSphere) {
-                float t;
-                if (sphere_hit(r, v0.x, v0.y, v0.z, v1.x, t) && t >= r.tmin) {
-                    if (ANY) {
-                        if (t < r.tmax_eff)
-                            return true;
-                    } else if (better(t, prio_other(id), best)) {
-                        sphere_uv(r, v0.x, v0.y, v0.z, t, best.u, best.v);
-                        best.t = t;
-                        best.prim = prio_other(id);
-                        best.tcull = cull_limit(t);
-                        if (best_rec)
-                            *best_rec = i;
-                    }
-                }
-            } else {
-                float t, u, v;
-                if (cube_hit(r, v0, v1, t, u, v)) {
-                    if (ANY) {
-                        if (t < r.tmax_eff)
-                            return true;
-                    } else if (better(t, prio_cube(id), best)) {
-                        best.t = t;
-                        best.u = u;
-                        best.v = v;
-                        best.prim = prio_cube(id);
-                        best.tcull = cull_limit(t);
-                        if (best_rec)
-                            *best_rec = i;
-                    }
-                }
-            }
-        }
+        if (test_record_mixed<ANY>(v0, v1, v2, i, r, best, best_rec) && ANY)
+            return true;
         if (__float_as_uint(v1.w))
             break;
         ++i;

@@ -365,7 +365,8 @@ typedef struct igxrt_launch_params {
                              deeper entries spill to local memory; 0 = 16 */
     uint32_t packet_size; /* rays a warp claims per queue fetch: a multiple of
                              8 up to 4096; 0 = 16 */
-    uint32_t layout;      /* IGXRT_LAYOUT_* */
+    uint32_t layout;      /* IGXRT_LAYOUT_*; BVH2 and BVH4 launches trace the engine's own quantized
+                             form of the BVH4 nodes instead where the scene has one (same hits) */
     uint32_t ctas_per_sm; /* persistent CTAs per SM, 0 = as many as fit */
     uint32_t refill_lanes;/* a warp refetches rays once this many of its lanes
                              are idle (1..32); 0 = 8 */
@@ -669,8 +670,9 @@ igxrt_status igxrt_sync(igxrt_context* ctx, void* stream);
 
 /*
  * Instrumented traversal: per ray, the number of node records and primitive
- * records the closest (mode 0) or any-hit (mode 1) kernel fetches.  Used for
- * the bytes-per-ray roofline; the traversal order is the production kernel's.
+ * records a closest (mode 0) or any-hit (mode 1) traversal of the named
+ * layout's nodes fetches (the exact nodes, also where launches trace the
+ * scene's quantized form of BVH4).  Used for the bytes-per-ray roofline.
  */
 igxrt_status igxrt_count_fetches(igxrt_context* ctx, const igxrt_scene* scene,
                                  const igxrt_ray* rays, const uint32_t* prev_hit,
