@@ -314,15 +314,4 @@ struct NodeOps<IGXRT_LAYOUT_BVH4> {
     }
 };
 
-template <int LAYOUT>
-__device__ int interior_children(const typename NodeOps<LAYOUT>::Node* node) {
-    using Ops = NodeOps<LAYOUT>;
-    float f[Ops::kFloats];
-    Ops::load(node, f);
-    int k = 0;
-    for (int c = 0; c < Ops::kSlots; ++c)
-        k += (!Ops::empty(f, c) && Ops::child(f, c) >= 0) ? 1 : 0;
-    return k;
-}
-
 }  // namespace igxrt

@@ -3,27 +3,28 @@
 // The reference uploads its scene every frame (test/scene/niels_scene.cpp:
 // 61-70) and traces it with a linear loop; the host SAH builder takes about a
 // second per million triangles, so a per-frame scene needs a device build.
-// This is a linear BVH (Morton order + radix tree, after Karras 2012, "Maximizing
-// parallelism in the construction of BVHs, octrees, and k-d trees"), emitted in
-// the same node formats, records and padding rule as the host builder so that
-// the traversal kernels, the refit and the read-back work on it unchanged:
+// This is a linear BVH (Morton order, then the radix tree over the keys, built
+// bottom-up together with its boxes after Apetrei 2014, "Fast and Simple
+// Agglomerative LBVH Construction"), emitted in the same node formats, records
+// and padding rule as the host builder so that the traversal kernels, the
+// refit and the read-back work on it unchanged:
 //   1. scan: object bounds, max |coordinate|, scene and centroid boxes, the
 //      non-finite check (shared with the refit);
 //   2. keys: 30-bit Morton code of the centroid in the centroid box, above the
 //      object id (so keys are unique), sorted with CUB's radix sort;
-//   3. radix tree: one thread per internal node finds its range and split
-//      from the common-prefix lengths of neighbouring keys;
-//   4. boxes: one thread per object climbs from its leaf; at each node the
-//      first arriving child's thread stops and the second computes the union
-//      (nothing waits);
-//   5. leaves: a subtree of at most `max_leaf_size` objects becomes one leaf
+//   3. climb: one thread per object writes its record and climbs from its
+//      leaf; a node joins its neighbour across the boundary whose keys differ
+//      in the lower bit, and at each parent the first arriving child's thread
+//      stops and the second goes on with the union of both (nothing waits);
+//   4. leaves: a subtree of at most `max_leaf_size` objects becomes one leaf
 //      (its objects are contiguous in key order, so records stay in leaf
 //      order); the remaining internal nodes are compacted by a prefix sum and
 //      written as BVH2 nodes with padded boxes;
-//   6. BVH4: collapsed top down one level per launch, opening the child of
-//      largest area until four slots are used (the host rule);
-//   7. stack bounds and depth: bottom-up climbs like the refit's.
-// The scene is then allocated exactly and the arrays are copied into it.
+//   5. BVH4: collapsed top down one level per launch, opening the child of
+//      largest area until four slots are used (the host's choice); the levels
+//      carry the traversal-stack bounds and the depth along the paths.
+// The scene is then allocated exactly, the arrays are copied into it and its
+// grid nodes are written.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -37,11 +38,15 @@ using namespace igxrt;
 namespace {
 
 // State words after the scan's (which use 0..13).
-constexpr int kWordNodes2 = 16, kWordNodes4 = 17, kWordLeaves = 18, kWordStack2 = 19, kWordStack4 = 20,
-              kWordDepth = 21, kWordMalformed = 22;
+constexpr int kWordNodes2 = 16, kWordRoot = 17, kWordLeaves = 18, kWordStack4 = 19, kWordDepth = 20,
+              kWordMalformed = 21;
 constexpr int kWordSah = 32;       // double (words 32, 33)
 constexpr int kWordLevels = 64;    // frontier sizes of the BVH4 levels
 constexpr int kMaxLevels = 64;     // > key bits: no path is longer
+// Levels launched over the whole GPU.  A tree over scattered objects has
+// about log4 of its leaves, 10 at 300K objects; an empty level costs 1.2 us,
+// and one block takes whatever levels are left (bvh4_rest_kernel).
+constexpr int kWideLevels = 20;
 constexpr int kStateWords = kWordLevels + kMaxLevels + 1;
 constexpr uint32_t kDefaultLeaf = 4;
 
@@ -52,12 +57,12 @@ struct BuildArgs {
     uint32_t idbits;  // low key bits holding the object id
     uint32_t* state;
     const uint64_t* keys;  // sorted
-    int32_t* kchild;       // 2 per internal node: >= 0 internal, < 0 ~key position
-    uint2* krange;         // first, last key position
-    uint32_t* kparent;     // per internal node
-    uint32_t* lparent;     // per key position
-    float* kbox;           // 6 per internal node: lo xyz, hi xyz (unpadded)
-    uint32_t* arrive;      // per internal node (reused by the climbs)
+    // Internal node p splits its keys between positions p and p + 1.  Four
+    // float4 per node: the left child {lo, ref}{hi, first key position}, the
+    // right child {lo, ref}{hi, last key position}; ref >= 0 is an internal
+    // node, < 0 ~key position
+    float4* slots;
+    uint32_t* arrive;      // per internal node
     uint32_t* live;        // per internal node: 1 if it becomes a BVH2 node
     uint32_t* map;         // exclusive prefix sum of `live`
     igxrt_bvh2_node* nodes2;
@@ -65,9 +70,7 @@ struct BuildArgs {
     uint32_t* parents2;
     uint32_t* parents4;
     igxrt_prim_record* prims;
-    uint2* frontier[2];    // (BVH2 node, BVH4 node) pairs of one level
-    uint32_t* stack_v;     // climb values per node: stack bound
-    uint32_t* depth_v;     //                         depth
+    uint2* frontier[2];    // one level's {BVH2 node, stack entries above it | depth << 16}
 };
 
 __device__ __forceinline__ float key_float(uint32_t k) {
@@ -113,169 +116,139 @@ __global__ void morton_kernel(BuildArgs a, uint64_t* keys) {
     keys[id] = ((uint64_t)code << a.idbits) | id;
 }
 
-__device__ __forceinline__ int prefix(const uint64_t* keys, int64_t n, int64_t i, int64_t j) {
-    if (j < 0 || j >= n)
-        return -1;
-    return __clzll(keys[i] ^ keys[j]);
+__device__ __forceinline__ Box slot_box(const float4& lo, const float4& hi) {
+    return {{lo.x, lo.y, lo.z}, {hi.x, hi.y, hi.z}};
 }
 
-// Radix tree over the sorted keys (Karras 2012, section 4).
-__global__ void radix_tree_kernel(BuildArgs a) {
-    const int64_t n = a.n;
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n - 1)
-        return;
-    const uint64_t* k = a.keys;
-    const int d = prefix(k, n, i, i + 1) - prefix(k, n, i, i - 1) >= 0 ? 1 : -1;
-    const int dmin = prefix(k, n, i, i - d);
-    int64_t lmax = 2;
-    while (prefix(k, n, i, i + lmax * d) > dmin)
-        lmax <<= 1;
-    int64_t l = 0;
-    for (int64_t t = lmax >> 1; t >= 1; t >>= 1)
-        if (prefix(k, n, i, i + (l + t) * d) > dmin)
-            l += t;
-    const int64_t j = i + l * d;
-    const int dnode = prefix(k, n, i, j);
-    int64_t s = 0, t = l;
-    do {
-        t = (t + 1) >> 1;
-        if (prefix(k, n, i, i + (s + t) * d) > dnode)
-            s += t;
-    } while (t > 1);
-    const int64_t g = i + s * d + min(d, 0);
-    const int64_t first = min(i, j), last = max(i, j);
-    const int32_t left = first == g ? ~(int32_t)g : (int32_t)g;
-    const int32_t right = last == g + 1 ? ~(int32_t)(g + 1) : (int32_t)(g + 1);
-    a.kchild[2 * i] = left;
-    a.kchild[2 * i + 1] = right;
-    a.krange[i] = make_uint2((uint32_t)first, (uint32_t)last);
-    if (left >= 0)
-        a.kparent[left] = (uint32_t)i;
-    else
-        a.lparent[~left] = (uint32_t)i;
-    if (right >= 0)
-        a.kparent[right] = (uint32_t)i;
-    else
-        a.lparent[~right] = (uint32_t)i;
-    if (i == 0)
-        a.kparent[0] = kNoParent;
-}
-
-__device__ Box child_box(const BuildArgs& a, int32_t ref) {
-    Box b;
-    if (ref < 0)
-        return object_box<false>(a.obj, object_of(a, (uint32_t)~ref));
-    const float2* p = reinterpret_cast<const float2*>(a.kbox + 6 * (size_t)ref);
-    const float2 x = __ldcg(p), y = __ldcg(p + 1), z = __ldcg(p + 2);
-    b.lo[0] = x.x;
-    b.lo[1] = x.y;
-    b.lo[2] = y.x;
-    b.hi[0] = y.y;
-    b.hi[1] = z.x;
-    b.hi[2] = z.y;
-    return b;
-}
-
-// Bottom-up boxes: the second child to arrive at a node computes its box.
-__global__ void radix_boxes_kernel(BuildArgs a) {
-    const uint32_t leaf = blockIdx.x * blockDim.x + threadIdx.x;
-    if (leaf >= a.n)
-        return;
-    uint32_t p = a.lparent[leaf];
-    for (int steps = 0; p != kNoParent; ++steps) {
-        if (steps >= kMaxLevels) {  // deeper than the key bits allow: malformed
-            atomicOr(a.state + kWordMalformed, 1u);
-            return;
-        }
-        if (arrive_at(a.arrive + p) == 0)
-            return;  // the sibling's thread computes this node
-        Box b = child_box(a, a.kchild[2 * p]);
-        b.grow(child_box(a, a.kchild[2 * p + 1]));
-        float* o = a.kbox + 6 * (size_t)p;
-        o[0] = b.lo[0];
-        o[1] = b.lo[1];
-        o[2] = b.lo[2];
-        o[3] = b.hi[0];
-        o[4] = b.hi[1];
-        o[5] = b.hi[2];
-        p = a.kparent[p];
-    }
-}
-
-__device__ __forceinline__ uint32_t range_count(const BuildArgs& a, uint32_t node) {
-    const uint2 r = a.krange[node];
-    return r.y - r.x + 1;
-}
-
-__global__ void live_kernel(BuildArgs a) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < a.n - 1)
-        a.live[i] = range_count(a, i) > a.leaf ? 1u : 0u;
-}
-
-// Records in key order (leaf_end is set when the leaves are emitted).
-__global__ void build_records_kernel(BuildArgs a) {
+// Records in key order (leaf_end is set when the leaves are emitted), and the
+// tree with its boxes.  A climber's step is a release of the 32 bytes it hands
+// to its parent, the arrival, and one load of its sibling's 32 bytes; its own
+// box stays in registers.  For 300K random triangles this pass takes 82 us (cold),
+// where records, radix tree and boxes as three kernels took 22 + 20 + 51 us.
+__global__ void climb_kernel(BuildArgs a) {
     const uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x;
     if (pos >= a.n)
         return;
     const uint32_t id = object_of(a, pos);
-    igxrt_prim_record r{};
-    fill_record(a.obj, id, r);
-    r.prim = id;
-    r.leaf_end = 0;
-    r.pad = id < a.obj.nt ? kPrimTriangle : (id < a.obj.nt + a.obj.ns ? kPrimSphere : kPrimCube);
-    a.prims[pos] = r;
+    igxrt_prim_record rec{};
+    fill_record(a.obj, id, rec);
+    rec.prim = id;
+    rec.leaf_end = 0;
+    rec.pad = id < a.obj.nt ? kPrimTriangle : (id < a.obj.nt + a.obj.ns ? kPrimSphere : kPrimCube);
+    a.prims[pos] = rec;
+    Box box = object_box<false>(a.obj, id);
+    uint32_t first = pos, last = pos;
+    int32_t ref = ~(int32_t)pos;
+    for (int steps = 0; first != 0 || last != a.n - 1; ++steps) {
+        if (steps >= kMaxLevels) {  // deeper than the key bits allow: malformed
+            atomicOr(a.state + kWordMalformed, 1u);
+            return;
+        }
+        // the keys are unique, so the two boundaries' differences never tie
+        const uint64_t below = first > 0 ? a.keys[first - 1] ^ a.keys[first] : ~0ull;
+        const uint64_t above = last < a.n - 1 ? a.keys[last] ^ a.keys[last + 1] : ~0ull;
+        const bool left = above < below;  // the left child of the node that splits at `last`
+        const uint32_t p = left ? last : first - 1;
+        float4* own = a.slots + 4 * (size_t)p + (left ? 0 : 2);
+        own[0] = make_float4(box.lo[0], box.lo[1], box.lo[2], __int_as_float(ref));
+        own[1] = make_float4(box.hi[0], box.hi[1], box.hi[2], __uint_as_float(left ? first : last));
+        if (arrive_at(a.arrive + p) == 0)
+            return;  // the sibling's thread goes on
+        const float4* other = a.slots + 4 * (size_t)p + (left ? 2 : 0);
+        const float4 lo = __ldcg(other), hi = __ldcg(other + 1);
+        Box sibling = slot_box(lo, hi);
+        if (left) {
+            box.grow(sibling);
+            last = __float_as_uint(hi.w);
+        } else {
+            sibling.grow(box);
+            box = sibling;
+            first = __float_as_uint(hi.w);
+        }
+        a.live[p] = last - first + 1 > a.leaf ? 1u : 0u;
+        ref = (int32_t)p;
+    }
+    if (a.n > 1)
+        a.state[kWordRoot] = (uint32_t)ref;
 }
 
-__device__ __forceinline__ void put_slot2(igxrt_bvh2_node& o, int c, const Box& b, int32_t ref) {
-    NodeOps<IGXRT_LAYOUT_BVH2>::put(&o, c, b);
-    o.child[c] = ref;
+// The BVH2 node of a live internal node: the prefix sum's place, with the
+// root's and the first one's exchanged (traversals start at node 0).
+__device__ __forceinline__ uint32_t node2_of(const BuildArgs& a, uint32_t i, uint32_t root) {
+    const uint32_t m = a.map[i];
+    return i == root ? 0u : (m == 0u ? a.map[root] : m);
 }
 
 // BVH2 nodes from the live internal nodes.  Sums the SAH cost (areas relative
-// to the root box; node cost 1, object cost 1, as the host builder's default).
-__global__ void emit2_kernel(BuildArgs a) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+// to the root box; node cost 1, object cost 1, as the host builder's default),
+// one double atomic per block of a grid of at most a few rounds.
+__global__ void __launch_bounds__(256) emit2_kernel(BuildArgs a) {
+    if (a.state[kWordMalformed])
+        return;  // slots may be unwritten
     double sah = 0.0;
     uint32_t leaves = 0;
-    if (i < a.n - 1 && a.live[i]) {
-        const float pad = box_pad(a.state);
-        const float root_area = child_box(a, 0).half_area();
-        const float inv_root = root_area > 0.f ? 1.f / root_area : 0.f;
-        const uint32_t node = a.map[i];
+    const uint32_t root = a.state[kWordRoot];
+    const float4* rs = a.slots + 4 * (size_t)root;
+    Box rb = slot_box(rs[0], rs[1]);
+    rb.grow(slot_box(rs[2], rs[3]));
+    const float root_area = rb.half_area();
+    const float inv_root = root_area > 0.f ? 1.f / root_area : 0.f;
+    const float pad = box_pad(a.state);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n - 1; i += gridDim.x * blockDim.x) {
+        if (!a.live[i])
+            continue;
+        const uint32_t node = node2_of(a, i, root);
+        const float4* s = a.slots + 4 * (size_t)i;
         igxrt_bvh2_node o{};
-        sah += root_area > 0.f ? (double)child_box(a, (int32_t)i).half_area() * inv_root : 1.0;
+        Box both;
+        both.reset();
         for (int c = 0; c < 2; ++c) {
-            const int32_t ref = a.kchild[2 * i + c];
-            Box b = child_box(a, ref);
+            const float4 lo = s[2 * c], hi = s[2 * c + 1];
+            Box b = slot_box(lo, hi);
+            both.grow(b);
             const float rel = root_area > 0.f ? b.half_area() * inv_root : 1.f;
+            const int32_t ref = __float_as_int(lo.w);
             b.pad(pad);
+            NodeOps<IGXRT_LAYOUT_BVH2>::put(&o, c, b);
             if (ref >= 0 && a.live[ref]) {
-                const uint32_t child = a.map[ref];
-                put_slot2(o, c, b, (int32_t)child);
+                const uint32_t child = node2_of(a, (uint32_t)ref, root);
+                o.child[c] = (int32_t)child;
                 a.parents2[child] = node;
             } else {
-                const uint2 r = ref >= 0 ? a.krange[ref] : make_uint2(~ref, ~ref);
-                put_slot2(o, c, b, ~(int32_t)r.x);
-                a.prims[r.y].leaf_end = 1;
-                sah += (double)rel * (r.y - r.x + 1);
+                const uint32_t bound = __float_as_uint(hi.w);
+                const uint32_t first = c == 0 ? bound : i + 1, last = c == 0 ? i : bound;
+                o.child[c] = ~(int32_t)first;
+                a.prims[last].leaf_end = 1;
+                sah += (double)rel * (last - first + 1);
                 ++leaves;
             }
         }
+        sah += root_area > 0.f ? (double)both.half_area() * inv_root : 1.0;
         a.nodes2[node] = o;
-        if (i == 0) {
+        if (i == root) {
             a.parents2[0] = kNoParent;
             a.state[kWordNodes2] = a.map[a.n - 2] + a.live[a.n - 2];
         }
     }
-    // one atomic per warp
+    __shared__ double block_sah[8];
+    __shared__ uint32_t block_leaves[8];
     leaves = __reduce_add_sync(0xffffffffu, leaves);
     for (int off = 16; off > 0; off >>= 1)
         sah += __shfl_down_sync(0xffffffffu, sah, off);
-    if ((threadIdx.x & 31) == 0 && leaves) {
-        atomicAdd(a.state + kWordLeaves, leaves);
-        atomicAdd(reinterpret_cast<double*>(a.state + kWordSah), sah);
+    if ((threadIdx.x & 31) == 0) {
+        block_sah[threadIdx.x / 32] = sah;
+        block_leaves[threadIdx.x / 32] = leaves;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) {
+            sah += block_sah[w];
+            leaves += block_leaves[w];
+        }
+        if (leaves) {
+            atomicAdd(a.state + kWordLeaves, leaves);
+            atomicAdd(reinterpret_cast<double*>(a.state + kWordSah), sah);
+        }
     }
 }
 
@@ -283,14 +256,22 @@ __global__ void emit2_kernel(BuildArgs a) {
 // slot 0 (the host builder's layout for a one-leaf tree).
 __global__ void emit_single_leaf_kernel(BuildArgs a) {
     const float pad = box_pad(a.state);
-    Box b = a.n == 1 ? child_box(a, ~0) : child_box(a, 0);
+    Box b;
+    if (a.n == 1) {
+        b = object_box<false>(a.obj, object_of(a, 0));
+    } else {
+        const float4* s = a.slots + 4 * (size_t)a.state[kWordRoot];
+        b = slot_box(s[0], s[1]);
+        b.grow(slot_box(s[2], s[3]));
+    }
     b.pad(pad);
     igxrt_bvh2_node o{};
-    put_slot2(o, 0, b, ~0);
+    NodeOps<IGXRT_LAYOUT_BVH2>::put(&o, 0, b);
+    o.child[0] = ~0;
     Box e;
     for (int k = 0; k < 3; ++k)
         e.lo[k] = e.hi[k] = INFINITY;
-    put_slot2(o, 1, e, 0);
+    NodeOps<IGXRT_LAYOUT_BVH2>::put(&o, 1, e);
     a.nodes2[0] = o;
     a.parents2[0] = kNoParent;
     igxrt_bvh4_node q{};
@@ -302,137 +283,173 @@ __global__ void emit_single_leaf_kernel(BuildArgs a) {
     a.parents4[0] = kNoParent;
     a.prims[a.n - 1].leaf_end = 1;
     a.state[kWordNodes2] = 1;
-    a.state[kWordNodes4] = 1;
+    a.state[kWordLevels] = 1;
     a.state[kWordLeaves] = 1;
+    a.state[kWordDepth] = 1;
     *reinterpret_cast<double*>(a.state + kWordSah) = (double)a.n;
 }
 
 __global__ void bvh4_root_kernel(BuildArgs a) {
     a.frontier[0][0] = make_uint2(0, 0);
-    a.state[kWordLevels] = 1;
-    a.state[kWordNodes4] = 1;
+    a.state[kWordLevels] = a.state[kWordMalformed] ? 0u : 1u;
     a.parents4[0] = kNoParent;
 }
 
 // One BVH4 level: each frontier BVH2 node becomes a BVH4 node whose slots are
 // its descendants, opened largest-area-first until four slots are used.  The
-// levels are chained by programmatic dependent launch: the next level's blocks
-// are scheduled as soon as this one starts, and its griddepcontrol.wait
-// returns once this grid has finished and its writes are visible, so the
-// (mostly empty) deep levels cost no launch gap.
-__global__ void emit4_level_kernel(BuildArgs a, int level) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;");
-    const uint32_t count = a.state[kWordLevels + level];
+// level's nodes follow the earlier levels' in frontier order, so a node's
+// place and its parent's need no counter of their own: a warp takes places in
+// the next level for all its children with one atomic (two atomics per child
+// before, and two climbs over the finished trees, 40 + 32 us, for the stack
+// bounds and the depth).  Along a path the
+// frontier carries the stack entries a traversal may hold on arrival (each
+// node above pushes its used slots minus one) and the BVH2 depth; every BVH2
+// node is opened by exactly one BVH4 node, so the maxima cover the tree.
+// Called by whole warps with the same arguments.  Returns the level's size.
+__device__ uint32_t emit4_level(const BuildArgs& a, int level, uint32_t thread, uint32_t threads) {
+    const uint32_t lane = threadIdx.x & 31u, lower = (1u << lane) - 1u;
+    const uint32_t* counts = a.state + kWordLevels;
+    const uint32_t count = __ldcg(counts + level);
+    if (count == 0)
+        return 0;
+    uint32_t base = (int)lane < level ? __ldcg(counts + lane) : 0u;
+    if ((int)lane + 32 < level)
+        base += __ldcg(counts + lane + 32);
+    base = __reduce_add_sync(0xffffffffu, base);  // nodes of the earlier levels
     const uint2* in = a.frontier[level & 1];
     uint2* out = a.frontier[(level + 1) & 1];
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
-        const uint2 job = in[t];
+    uint32_t deepest = 0, stack = 0;
+    for (uint32_t t0 = thread & ~31u; t0 < count; t0 += threads) {
+        const uint32_t t = t0 + lane;
+        const bool mine = t < count;
         Box box[4];
         int32_t ref[4];
-        float area[4];
+        uint32_t depth[4];  // of the BVH2 node that holds the slot
         int used = 0;
-        using Ops2 = NodeOps<IGXRT_LAYOUT_BVH2>;
-        float f[Ops2::kFloats];
-        Ops2::load(a.nodes2 + job.x, f);
-        for (int c = 0; c < 2; ++c) {
-            if (Ops2::empty(f, c))
-                continue;
-            Ops2::get(f, c, box[used]);
-            ref[used] = Ops2::child(f, c);
-            area[used] = box[used].half_area();
-            ++used;
-        }
-        while (used < 4) {
-            int pick = -1;
-            float best = -1.f;
-            for (int s = 0; s < used; ++s)
-                if (ref[s] >= 0 && area[s] > best) {
-                    best = area[s];
-                    pick = s;
+        uint32_t kids = 0, above = 0;
+        if (mine) {
+            const uint2 job = __ldcg(in + t);
+            float area[4];
+            using Ops2 = NodeOps<IGXRT_LAYOUT_BVH2>;
+            float f[Ops2::kFloats];
+            Ops2::load(a.nodes2 + job.x, f);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {  // the trees of this path have no empty BVH2 slot
+                Ops2::get(f, c, box[c]);
+                ref[c] = Ops2::child(f, c);
+                area[c] = box[c].half_area();
+                depth[c] = (job.y >> 16) + 1u;
+            }
+            used = 2;
+            // the opened slot's first child takes its place, the second the
+            // next free slot: every index is fixed, so the slots stay in
+            // registers
+#pragma unroll
+            for (int free = 2; free < 4; ++free) {
+                if (used < free)
+                    break;
+                int pick = -1;
+                int32_t open = 0;
+                uint32_t d = 0;
+                float best = -1.f;
+#pragma unroll
+                for (int s = 0; s < free; ++s)
+                    if (ref[s] >= 0 && area[s] > best) {
+                        best = area[s];
+                        pick = s;
+                        open = ref[s];
+                        d = depth[s] + 1u;
+                    }
+                if (pick < 0)
+                    break;
+                Ops2::load(a.nodes2 + open, f);
+                Box b;
+                Ops2::get(f, 0, b);
+#pragma unroll
+                for (int s = 0; s < free; ++s)
+                    if (s == pick) {
+                        box[s] = b;
+                        ref[s] = Ops2::child(f, 0);
+                        area[s] = b.half_area();
+                        depth[s] = d;
+                    }
+                Ops2::get(f, 1, box[free]);
+                ref[free] = Ops2::child(f, 1);
+                area[free] = box[free].half_area();
+                depth[free] = d;
+                used = free + 1;
+            }
+            above = (job.y & 0xffffu) + (uint32_t)used - 1u;
+            stack = max(stack, above);
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+                if (s < used) {
+                    kids += ref[s] >= 0 ? 1u : 0u;
+                    deepest = max(deepest, depth[s]);
                 }
-            if (pick < 0)
-                break;
-            Ops2::load(a.nodes2 + ref[pick], f);
-            for (int s = used; s > pick + 1; --s) {  // make room after `pick`
-                box[s] = box[s - 1];
-                ref[s] = ref[s - 1];
-                area[s] = area[s - 1];
-            }
-            for (int c = 0; c < 2; ++c) {
-                Ops2::get(f, c, box[pick + c]);
-                ref[pick + c] = Ops2::child(f, c);
-                area[pick + c] = box[pick + c].half_area();
-            }
-            ++used;
         }
+        uint32_t place = 0, total = 0;
+        for (int k = 0; k < 3; ++k) {  // kids <= 4
+            const uint32_t b = __ballot_sync(0xffffffffu, (kids >> k) & 1u);
+            place += (uint32_t)__popc(b & lower) << k;
+            total += (uint32_t)__popc(b) << k;
+        }
+        uint32_t taken = 0;
+        if (lane == 0 && total)
+            taken = atomicAdd(a.state + kWordLevels + level + 1, total);
+        place += __shfl_sync(0xffffffffu, taken, 0);
+        if (!mine)
+            continue;
         igxrt_bvh4_node o{};
+#pragma unroll
         for (int s = 0; s < 4; ++s) {
             if (s < used) {
                 NodeOps<IGXRT_LAYOUT_BVH4>::put(&o, s, box[s]);
+                o.child[s] = ref[s];
                 if (ref[s] >= 0) {
-                    const uint32_t child = atomicAdd(a.state + kWordNodes4, 1u);
-                    a.parents4[child] = job.y;
-                    out[atomicAdd(a.state + kWordLevels + level + 1, 1u)] = make_uint2((uint32_t)ref[s], child);
+                    const uint32_t child = base + count + place;
+                    a.parents4[child] = base + t;
+                    out[place++] = make_uint2((uint32_t)ref[s], above | depth[s] << 16);
                     o.child[s] = (int32_t)child;
-                } else {
-                    o.child[s] = ref[s];
                 }
             } else {
                 Box e;
                 for (int k = 0; k < 3; ++k)
                     e.lo[k] = e.hi[k] = INFINITY;
                 NodeOps<IGXRT_LAYOUT_BVH4>::put(&o, s, e);
-                o.child[s] = 0;
             }
         }
-        a.nodes4[job.y] = o;
+        a.nodes4[base + t] = o;
     }
+    stack = __reduce_max_sync(0xffffffffu, stack);
+    deepest = __reduce_max_sync(0xffffffffu, deepest);
+    if (lane == 0) {  // the words soon hold the maxima: most warps only read them
+        if (stack > __ldcg(a.state + kWordStack4))
+            atomicMax(a.state + kWordStack4, stack);
+        if (deepest > __ldcg(a.state + kWordDepth))
+            atomicMax(a.state + kWordDepth, deepest);
+    }
+    return count;
 }
 
-// Exact traversal-stack bound (a node pushes its entered slots minus one) and
-// depth, bottom-up through the parent links like the refit.
-template <int LAYOUT>
-__global__ void stack_bound_kernel(BuildArgs a, uint32_t count) {
-    using Ops = NodeOps<LAYOUT>;
-    using Node = typename Ops::Node;
-    const Node* nodes = LAYOUT == IGXRT_LAYOUT_BVH2 ? (const Node*)a.nodes2 : (const Node*)a.nodes4;
-    const uint32_t* parents = LAYOUT == IGXRT_LAYOUT_BVH2 ? a.parents2 : a.parents4;
-    uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
-    if (node >= count || interior_children<LAYOUT>(nodes + node) != 0)
-        return;
-    for (int steps = 0;; ++steps) {
-        if (steps > kMaxLevels) {
-            atomicOr(a.state + kWordMalformed, 2u);
+// The wide levels, chained by programmatic dependent launch: the next level's
+// blocks are scheduled as soon as this one starts, and its
+// griddepcontrol.wait returns once this grid has finished and its writes are
+// visible, so an empty level costs no launch gap.
+__global__ void __launch_bounds__(256) emit4_level_kernel(BuildArgs a, int level) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+    emit4_level(a, level, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+// The levels after them, one block: empty but for deep trees, whose last
+// levels are mostly narrow.
+__global__ void __launch_bounds__(1024) bvh4_rest_kernel(BuildArgs a) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int level = kWideLevels; level < kMaxLevels; ++level) {
+        if (emit4_level(a, level, threadIdx.x, blockDim.x) == 0)
             return;
-        }
-        float f[Ops::kFloats];
-        Ops::load(nodes + node, f);
-        uint32_t deepest = 0, depth = 0;
-        int used = 0;
-        for (int c = 0; c < Ops::kSlots; ++c) {
-            if (Ops::empty(f, c))
-                continue;
-            ++used;
-            const int32_t ch = Ops::child(f, c);
-            if (ch >= 0) {
-                deepest = max(deepest, __ldcg(a.stack_v + ch));
-                depth = max(depth, __ldcg(a.depth_v + ch));
-            }
-        }
-        a.stack_v[node] = deepest + (used ? used - 1 : 0);
-        a.depth_v[node] = depth + 1;
-        const uint32_t p = parents[node];
-        if (p == kNoParent) {
-            a.state[LAYOUT == IGXRT_LAYOUT_BVH2 ? kWordStack2 : kWordStack4] = a.stack_v[node];
-            if (LAYOUT == IGXRT_LAYOUT_BVH2)
-                a.state[kWordDepth] = a.depth_v[node];
-            return;
-        }
-        const uint32_t need = (uint32_t)interior_children<LAYOUT>(nodes + p);
-        if (arrive_at(a.arrive + p) + 1u != need)
-            return;
-        node = p;
+        __syncthreads();
     }
 }
 
@@ -482,7 +499,7 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
     // CUB scratch sizes
     size_t sort_bytes = 0, scan_bytes = 0;
     cub::DoubleBuffer<uint64_t> keys_db(nullptr, nullptr);
-    cudaError_t e = cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, keys_db, (int)nl, 0,
+    cudaError_t e = cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, keys_db, (int)nl, (int)a.idbits,
                                                     30 + (int)a.idbits, s);
     if (e == cudaSuccess)
         e = cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
@@ -492,9 +509,9 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
 
     // one scratch allocation, 256-byte aligned parts
     std::vector<size_t> sizes = {
-        kStateWords * 4, 2 * nl * 8, 2 * ni * 4, ni * 8, ni * 4, nl * 4, 6 * ni * 4, ni * 4, ni * 4,
-        ni * 4, ni * sizeof(igxrt_bvh2_node), ni * sizeof(igxrt_bvh4_node), ni * 4, ni * 4,
-        nl * sizeof(igxrt_prim_record), 2 * ni * 8, ni * 4, ni * 4, std::max(sort_bytes, scan_bytes)};
+        kStateWords * 4, 2 * nl * 8, 4 * ni * sizeof(float4), ni * 4, ni * 4, ni * 4,
+        ni * sizeof(igxrt_bvh2_node), ni * sizeof(igxrt_bvh4_node), ni * 4, ni * 4,
+        nl * sizeof(igxrt_prim_record), 2 * ni * 8, std::max(sort_bytes, scan_bytes)};
     std::vector<size_t> offs(sizes.size());
     size_t total = 0;
     for (size_t k = 0; k < sizes.size(); ++k) {
@@ -511,11 +528,7 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
     a.state = next((uint32_t*)nullptr);
     uint64_t* keys0 = next((uint64_t*)nullptr);
     uint64_t* keys1 = keys0 + nl;
-    a.kchild = next((int32_t*)nullptr);
-    a.krange = next((uint2*)nullptr);
-    a.kparent = next((uint32_t*)nullptr);
-    a.lparent = next((uint32_t*)nullptr);
-    a.kbox = next((float*)nullptr);
+    a.slots = next((float4*)nullptr);
     a.arrive = next((uint32_t*)nullptr);
     a.live = next((uint32_t*)nullptr);
     a.map = next((uint32_t*)nullptr);
@@ -526,8 +539,6 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
     a.prims = next((igxrt_prim_record*)nullptr);
     a.frontier[0] = next((uint2*)nullptr);
     a.frontier[1] = a.frontier[0] + ni;
-    a.stack_v = next((uint32_t*)nullptr);
-    a.depth_v = next((uint32_t*)nullptr);
     void* cub_temp = base + offs[part++];
 
     const uint32_t threads = 256;
@@ -543,25 +554,23 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
     if (n) {
         morton_kernel<<<blocks(n), threads, 0, s>>>(a, keys0);
         keys_db = cub::DoubleBuffer<uint64_t>(keys0, keys1);
-        e = cub::DeviceRadixSort::SortKeys(cub_temp, sort_bytes, keys_db, (int)n, 0, 30 + (int)a.idbits, s);
+        // by the code bits alone: the keys go in by ascending id and the sort
+        // is stable (four passes instead of seven at 300K objects, -33 us)
+        e = cub::DeviceRadixSort::SortKeys(cub_temp, sort_bytes, keys_db, (int)n, (int)a.idbits,
+                                           30 + (int)a.idbits, s);
         if (e != cudaSuccess)
             return cuda_fail(ctx, e, "key sort");
         a.keys = keys_db.Current();
-        build_records_kernel<<<blocks(n), threads, 0, s>>>(a);
-    }
-    if (n > 1) {
-        radix_tree_kernel<<<blocks(n - 1), threads, 0, s>>>(a);
-        radix_boxes_kernel<<<blocks(n), threads, 0, s>>>(a);
+        climb_kernel<<<blocks(n), threads, 0, s>>>(a);
     }
     const bool single = n >= 1 && n <= leaf;
     if (single) {
         emit_single_leaf_kernel<<<1, 1, 0, s>>>(a);
     } else if (n > 1) {
-        live_kernel<<<blocks(n - 1), threads, 0, s>>>(a);
         e = cub::DeviceScan::ExclusiveSum(cub_temp, scan_bytes, a.live, a.map, (int)(n - 1), s);
         if (e != cudaSuccess)
             return cuda_fail(ctx, e, "node compaction");
-        emit2_kernel<<<blocks(n - 1), threads, 0, s>>>(a);
+        emit2_kernel<<<std::min<uint32_t>(blocks(n - 1), (uint32_t)std::max(ctx->sm_count, 1) * 8), threads, 0, s>>>(a);
         bvh4_root_kernel<<<1, 1, 0, s>>>(a);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((uint32_t)std::max(ctx->sm_count, 1) * 4);
@@ -572,8 +581,12 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        for (int level = 0; level < kMaxLevels && e == cudaSuccess; ++level)
+        for (int level = 0; level < kWideLevels && e == cudaSuccess; ++level)
             e = cudaLaunchKernelEx(&cfg, emit4_level_kernel, a, level);
+        cfg.gridDim = dim3(1);
+        cfg.blockDim = dim3(1024);
+        if (e == cudaSuccess)
+            e = cudaLaunchKernelEx(&cfg, bvh4_rest_kernel, a);
         if (e != cudaSuccess)
             return cuda_fail(ctx, e, "BVH4 level launch");
     }
@@ -589,32 +602,14 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
         return fail(ctx, IGXRT_ERROR_INVALID_ARGUMENT, non_finite_message(w[kWordBad], n));
     if (w[kWordMalformed])
         return fail(ctx, IGXRT_ERROR_INVALID_BVH, "GPU build: malformed radix tree");
-    const uint32_t n2 = n ? w[kWordNodes2] : 0, n4 = n ? w[kWordNodes4] : 0;
+    const uint32_t n2 = n ? w[kWordNodes2] : 0;
+    uint32_t n4 = 0;
+    for (int level = 0; level <= kMaxLevels; ++level)
+        n4 += w[kWordLevels + level];
     if (w[kWordLevels + kMaxLevels] != 0)
         return fail(ctx, IGXRT_ERROR_INVALID_BVH, "GPU build: BVH4 deeper than the level limit");
     if (n2 > ni || n4 > ni)
         return fail(ctx, IGXRT_ERROR_INVALID_BVH, "GPU build: node count out of range");
-
-    // stack bounds and depth
-    if (n) {
-        e = cudaMemsetAsync(a.arrive, 0, ni * 4, s);
-        if (e == cudaSuccess)
-            stack_bound_kernel<IGXRT_LAYOUT_BVH2><<<blocks(n2), threads, 0, s>>>(a, n2);
-        if (e == cudaSuccess)
-            e = cudaMemsetAsync(a.arrive, 0, ni * 4, s);
-        if (e == cudaSuccess)
-            stack_bound_kernel<IGXRT_LAYOUT_BVH4><<<blocks(n4), threads, 0, s>>>(a, n4);
-        if (e == cudaSuccess)
-            e = cudaGetLastError();
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(w, a.state, sizeof(w), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess)
-            e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess)
-            return cuda_fail(ctx, e, "GPU build stack bounds");
-        if (w[kWordMalformed])
-            return fail(ctx, IGXRT_ERROR_INVALID_BVH, "GPU build: malformed tree");
-    }
 
     igxrt_bvh_info info{};
     info.triangle_count = a.obj.nt;
@@ -636,7 +631,8 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
         info.bounds[k] = n ? key_to_float(~w[kWordLo + k]) : 0.f;
         info.bounds[3 + k] = n ? key_to_float(w[kWordHi + k]) : 0.f;
     }
-    info.max_stack[IGXRT_LAYOUT_BVH2] = n ? w[kWordStack2] : 0;
+    // a BVH2 node pushes one entry, the root of a one-leaf tree none
+    info.max_stack[IGXRT_LAYOUT_BVH2] = n && !single ? w[kWordDepth] : 0;
     info.max_stack[IGXRT_LAYOUT_BVH4] = n ? w[kWordStack4] : 0;
     info.device_bytes = sizeof(igxrt_bvh2_node) * (uint64_t)n2 + sizeof(igxrt_bvh4_node) * (uint64_t)n4 +
                         sizeof(igxrt_prim_record) * (uint64_t)n + sizeof(igxrt_triangle) * (uint64_t)a.obj.nt +
