@@ -79,6 +79,14 @@ igxrt_status resolve_params(igxrt_context* ctx, const igxrt_launch_params& in, i
     return IGXRT_OK;
 }
 
+cudaError_t pool_alloc(igxrt_context* ctx, void** ptr, size_t bytes, cudaStream_t stream, bool& pooled) {
+    pooled = ctx->pool && cudaMallocFromPoolAsync(ptr, bytes, ctx->pool, stream) == cudaSuccess;
+    if (pooled)
+        return cudaSuccess;
+    cudaGetLastError();
+    return cudaMalloc(ptr, bytes);
+}
+
 // One device allocation per scene, 256-byte aligned sub-buffers in this
 // order: BVH2 nodes, BVH4 nodes, records, triangles, planes, parent links of
 // BVH2 and BVH4, refit words, BVH8 nodes, BVH8 slot sources, grid nodes, the
@@ -86,7 +94,7 @@ igxrt_status resolve_params(igxrt_context* ctx, const igxrt_launch_params& in, i
 // pointer and count of the scene from `info` and the node counts; the
 // contents are the caller's to write.
 igxrt_status allocate_scene(igxrt_context* ctx, const igxrt_bvh_info& info, uint32_t n2, uint32_t n4,
-                            uint32_t n8, igxrt_scene*& out) {
+                            uint32_t n8, igxrt_scene*& out, bool pool, cudaStream_t stream) {
     out = nullptr;
     igxrt_scene* s = new (std::nothrow) igxrt_scene();
     if (!s)
@@ -106,7 +114,8 @@ igxrt_status allocate_scene(igxrt_context* ctx, const igxrt_bvh_info& info, uint
     const size_t bs8 = round_up((size_t)n8 * 8 * sizeof(uint32_t), 256);
     const size_t o8 = b2 + b4 + bp + bt + bl + bpar + bw;
     const size_t og = o8 + b8 + bs8, bg = (size_t)n4 * 4 * sizeof(float4);
-    cudaError_t e = cudaMalloc(&s->d_mem, og + bg + 2 * sizeof(float4));
+    const size_t bytes = og + bg + 2 * sizeof(float4);
+    cudaError_t e = pool ? pool_alloc(ctx, &s->d_mem, bytes, stream, s->pooled) : cudaMalloc(&s->d_mem, bytes);
     if (e != cudaSuccess) {
         delete s;
         return cuda_fail(ctx, e, "scene allocation");
@@ -386,6 +395,17 @@ igxrt_status igxrt_create(int device, igxrt_context** out) {
         pageable = 0;
     }
     ctx->pageable_access = pageable != 0;
+    cudaMemPoolProps pool{};
+    pool.allocType = cudaMemAllocationTypePinned;
+    pool.location.type = cudaMemLocationTypeDevice;
+    pool.location.id = device;
+    uint64_t keep = kPoolKeep;
+    if (cudaMemPoolCreate(&ctx->pool, &pool) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->pool = nullptr;
+    } else if (cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+    }
     igxrt_launch_params defaults{};
     resolve_params(ctx, defaults, ctx->params);
     *out = ctx;
@@ -408,6 +428,8 @@ igxrt_status igxrt_destroy(igxrt_context* ctx) {
             cudaFree(ctx->d_stage);
         if (ctx->d_words)
             cudaFree(ctx->d_words);
+        if (ctx->pool)
+            cudaMemPoolDestroy(ctx->pool);  // scenes still alive keep their memory
     }
     delete ctx;
     return IGXRT_OK;
@@ -529,7 +551,10 @@ igxrt_status igxrt_scene_destroy(igxrt_scene* scene) {
     {
         DeviceGuard guard(scene->device);
         cudaDeviceSynchronize();
-        cudaFree(scene->d_mem);
+        if (scene->pooled)
+            cudaFreeAsync(scene->d_mem, nullptr);
+        else
+            cudaFree(scene->d_mem);
         cudaFree(scene->refit_boxes);
         cudaFree(scene->refit_unions);
     }

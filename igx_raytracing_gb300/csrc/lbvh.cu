@@ -453,10 +453,15 @@ __global__ void __launch_bounds__(1024) bvh4_rest_kernel(BuildArgs a) {
     }
 }
 
+// Build scratch, given back in stream order.
 struct Scratch {
     void* mem = nullptr;
+    bool pooled = false;
+    cudaStream_t stream = nullptr;
     ~Scratch() {
-        if (mem)
+        if (mem && pooled)
+            cudaFreeAsync(mem, stream);
+        else if (mem)
             cudaFree(mem);
     }
 };
@@ -519,7 +524,8 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
         total += round_up(std::max<size_t>(sizes[k], 1), 256);
     }
     Scratch scratch;
-    e = cudaMalloc(&scratch.mem, total);
+    scratch.stream = s;
+    e = pool_alloc(ctx, &scratch.mem, total, s, scratch.pooled);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "build scratch");
     char* base = static_cast<char*>(scratch.mem);
@@ -644,7 +650,7 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
                                kStackCapacity));
 
     igxrt_scene* scene = nullptr;
-    if ((st = allocate_scene(ctx, info, n2, n4, 0, scene)) != IGXRT_OK)
+    if ((st = allocate_scene(ctx, info, n2, n4, 0, scene, true, s)) != IGXRT_OK)
         return st;
     auto copy = [&](const void* dst, const void* src, size_t bytes) {
         if (e == cudaSuccess && bytes)
