@@ -265,16 +265,10 @@ struct NodeOps<IGXRT_LAYOUT_BVH2> {
         b.lo[2] = f[8 + 2 * c];
         b.hi[2] = f[8 + 2 * c + 1];
     }
+    // node arrays in device memory are 16-byte aligned
     __device__ static void put(Node* p, int c, const Box& b) {
-        float* x = c ? p->c1_x : p->c0_x;
-        float* y = c ? p->c1_y : p->c0_y;
-        float* z = c ? p->c1_z : p->c0_z;
-        x[0] = b.lo[0];
-        x[1] = b.hi[0];
-        y[0] = b.lo[1];
-        y[1] = b.hi[1];
-        z[0] = b.lo[2];
-        z[1] = b.hi[2];
+        reinterpret_cast<float4*>(p)[c] = make_float4(b.lo[0], b.hi[0], b.lo[1], b.hi[1]);
+        reinterpret_cast<float2*>(p)[4 + c] = make_float2(b.lo[2], b.hi[2]);
     }
 };
 

@@ -132,10 +132,11 @@ __global__ void climb_kernel(BuildArgs a) {
     const uint32_t id = object_of(a, pos);
     igxrt_prim_record rec{};
     fill_record(a.obj, id, rec);
-    rec.prim = id;
-    rec.leaf_end = 0;
-    rec.pad = id < a.obj.nt ? kPrimTriangle : (id < a.obj.nt + a.obj.ns ? kPrimSphere : kPrimCube);
-    a.prims[pos] = rec;
+    const uint32_t type = id < a.obj.nt ? kPrimTriangle : (id < a.obj.nt + a.obj.ns ? kPrimSphere : kPrimCube);
+    float4* out = reinterpret_cast<float4*>(a.prims + pos);
+    out[0] = make_float4(rec.p0[0], rec.p0[1], rec.p0[2], __uint_as_float(id));
+    out[1] = make_float4(rec.e1[0], rec.e1[1], rec.e1[2], 0.f);
+    out[2] = make_float4(rec.e2[0], rec.e2[1], rec.e2[2], __uint_as_float(type));
     Box box = object_box<false>(a.obj, id);
     uint32_t first = pos, last = pos;
     int32_t ref = ~(int32_t)pos;
@@ -199,7 +200,8 @@ __global__ void __launch_bounds__(256) emit2_kernel(BuildArgs a) {
             continue;
         const uint32_t node = node2_of(a, i, root);
         const float4* s = a.slots + 4 * (size_t)i;
-        igxrt_bvh2_node o{};
+        igxrt_bvh2_node* o = a.nodes2 + node;
+        int32_t refs[2];
         Box both;
         both.reset();
         for (int c = 0; c < 2; ++c) {
@@ -209,22 +211,22 @@ __global__ void __launch_bounds__(256) emit2_kernel(BuildArgs a) {
             const float rel = root_area > 0.f ? b.half_area() * inv_root : 1.f;
             const int32_t ref = __float_as_int(lo.w);
             b.pad(pad);
-            NodeOps<IGXRT_LAYOUT_BVH2>::put(&o, c, b);
+            NodeOps<IGXRT_LAYOUT_BVH2>::put(o, c, b);
             if (ref >= 0 && a.live[ref]) {
                 const uint32_t child = node2_of(a, (uint32_t)ref, root);
-                o.child[c] = (int32_t)child;
+                refs[c] = (int32_t)child;
                 a.parents2[child] = node;
             } else {
                 const uint32_t bound = __float_as_uint(hi.w);
                 const uint32_t first = c == 0 ? bound : i + 1, last = c == 0 ? i : bound;
-                o.child[c] = ~(int32_t)first;
+                refs[c] = ~(int32_t)first;
                 a.prims[last].leaf_end = 1;
                 sah += (double)rel * (last - first + 1);
                 ++leaves;
             }
         }
         sah += root_area > 0.f ? (double)both.half_area() * inv_root : 1.0;
-        a.nodes2[node] = o;
+        reinterpret_cast<int4*>(o)[3] = make_int4(refs[0], refs[1], 0, 0);
         if (i == root) {
             a.parents2[0] = kNoParent;
             a.state[kWordNodes2] = a.map[a.n - 2] + a.live[a.n - 2];
@@ -265,14 +267,12 @@ __global__ void emit_single_leaf_kernel(BuildArgs a) {
         b.grow(slot_box(s[2], s[3]));
     }
     b.pad(pad);
-    igxrt_bvh2_node o{};
-    NodeOps<IGXRT_LAYOUT_BVH2>::put(&o, 0, b);
-    o.child[0] = ~0;
     Box e;
     for (int k = 0; k < 3; ++k)
         e.lo[k] = e.hi[k] = INFINITY;
-    NodeOps<IGXRT_LAYOUT_BVH2>::put(&o, 1, e);
-    a.nodes2[0] = o;
+    NodeOps<IGXRT_LAYOUT_BVH2>::put(a.nodes2, 0, b);
+    NodeOps<IGXRT_LAYOUT_BVH2>::put(a.nodes2, 1, e);
+    reinterpret_cast<int4*>(a.nodes2)[3] = make_int4(~0, 0, 0, 0);
     a.parents2[0] = kNoParent;
     igxrt_bvh4_node q{};
     for (int c = 0; c < 4; ++c) {
@@ -400,26 +400,32 @@ __device__ uint32_t emit4_level(const BuildArgs& a, int level, uint32_t thread, 
         place += __shfl_sync(0xffffffffu, taken, 0);
         if (!mine)
             continue;
-        igxrt_bvh4_node o{};
+        Box b[4];
+        int32_t child[4];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
+            child[s] = 0;
             if (s < used) {
-                NodeOps<IGXRT_LAYOUT_BVH4>::put(&o, s, box[s]);
-                o.child[s] = ref[s];
+                b[s] = box[s];
+                child[s] = ref[s];
                 if (ref[s] >= 0) {
-                    const uint32_t child = base + count + place;
-                    a.parents4[child] = base + t;
+                    child[s] = (int32_t)(base + count + place);
+                    a.parents4[child[s]] = base + t;
                     out[place++] = make_uint2((uint32_t)ref[s], above | depth[s] << 16);
-                    o.child[s] = (int32_t)child;
                 }
             } else {
-                Box e;
                 for (int k = 0; k < 3; ++k)
-                    e.lo[k] = e.hi[k] = INFINITY;
-                NodeOps<IGXRT_LAYOUT_BVH4>::put(&o, s, e);
+                    b[s].lo[k] = b[s].hi[k] = INFINITY;
             }
         }
-        a.nodes4[base + t] = o;
+        float4* node = reinterpret_cast<float4*>(a.nodes4 + base + t);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            node[2 * k] = make_float4(b[0].lo[k], b[1].lo[k], b[2].lo[k], b[3].lo[k]);
+            node[2 * k + 1] = make_float4(b[0].hi[k], b[1].hi[k], b[2].hi[k], b[3].hi[k]);
+        }
+        reinterpret_cast<int4*>(node)[6] = make_int4(child[0], child[1], child[2], child[3]);
+        reinterpret_cast<int4*>(node)[7] = make_int4(0, 0, 0, 0);
     }
     stack = __reduce_max_sync(0xffffffffu, stack);
     deepest = __reduce_max_sync(0xffffffffu, deepest);
@@ -439,7 +445,11 @@ __device__ uint32_t emit4_level(const BuildArgs& a, int level, uint32_t thread, 
 __global__ void __launch_bounds__(256) emit4_level_kernel(BuildArgs a, int level) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
-    emit4_level(a, level, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    // consecutive warps of jobs go to consecutive blocks: a level of a few
+    // thousand nodes, each some forty 16-byte accesses to lines of its own,
+    // spreads over all SMs instead of filling the first blocks'
+    const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    emit4_level(a, level, warp * 32u + (threadIdx.x & 31u), gridDim.x * blockDim.x);
 }
 
 // The levels after them, one block: empty but for deep trees, whose last
