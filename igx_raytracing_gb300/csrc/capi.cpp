@@ -79,8 +79,16 @@ igxrt_status resolve_params(igxrt_context* ctx, const igxrt_launch_params& in, i
     return IGXRT_OK;
 }
 
+MemoryPool::~MemoryPool() {
+    if (!pool)
+        return;
+    DeviceGuard guard(device);
+    cudaDeviceSynchronize();  // frees queued into it
+    cudaMemPoolDestroy(pool);
+}
+
 cudaError_t pool_alloc(igxrt_context* ctx, void** ptr, size_t bytes, cudaStream_t stream, bool& pooled) {
-    pooled = ctx->pool && cudaMallocFromPoolAsync(ptr, bytes, ctx->pool, stream) == cudaSuccess;
+    pooled = ctx->pool && cudaMallocFromPoolAsync(ptr, bytes, ctx->pool->pool, stream) == cudaSuccess;
     if (pooled)
         return cudaSuccess;
     cudaGetLastError();
@@ -115,7 +123,10 @@ igxrt_status allocate_scene(igxrt_context* ctx, const igxrt_bvh_info& info, uint
     const size_t o8 = b2 + b4 + bp + bt + bl + bpar + bw;
     const size_t og = o8 + b8 + bs8, bg = (size_t)n4 * 4 * sizeof(float4);
     const size_t bytes = og + bg + 2 * sizeof(float4);
-    cudaError_t e = pool ? pool_alloc(ctx, &s->d_mem, bytes, stream, s->pooled) : cudaMalloc(&s->d_mem, bytes);
+    bool pooled = false;
+    cudaError_t e = pool ? pool_alloc(ctx, &s->d_mem, bytes, stream, pooled) : cudaMalloc(&s->d_mem, bytes);
+    if (pooled)
+        s->pool = ctx->pool;
     if (e != cudaSuccess) {
         delete s;
         return cuda_fail(ctx, e, "scene allocation");
@@ -400,11 +411,19 @@ igxrt_status igxrt_create(int device, igxrt_context** out) {
     pool.location.type = cudaMemLocationTypeDevice;
     pool.location.id = device;
     uint64_t keep = kPoolKeep;
-    if (cudaMemPoolCreate(&ctx->pool, &pool) != cudaSuccess) {
+    cudaMemPool_t handle = nullptr;
+    if (cudaMemPoolCreate(&handle, &pool) != cudaSuccess) {
         cudaGetLastError();
-        ctx->pool = nullptr;
-    } else if (cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-        cudaGetLastError();
+    } else {
+        if (cudaMemPoolSetAttribute(handle, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)
+            cudaGetLastError();  // keeps nothing: as cudaMalloc
+        try {
+            ctx->pool = std::make_shared<MemoryPool>();
+            ctx->pool->pool = handle;
+            ctx->pool->device = device;
+        } catch (const std::bad_alloc&) {
+            cudaMemPoolDestroy(handle);
+        }
     }
     igxrt_launch_params defaults{};
     resolve_params(ctx, defaults, ctx->params);
@@ -428,8 +447,6 @@ igxrt_status igxrt_destroy(igxrt_context* ctx) {
             cudaFree(ctx->d_stage);
         if (ctx->d_words)
             cudaFree(ctx->d_words);
-        if (ctx->pool)
-            cudaMemPoolDestroy(ctx->pool);  // scenes still alive keep their memory
     }
     delete ctx;
     return IGXRT_OK;
@@ -551,7 +568,7 @@ igxrt_status igxrt_scene_destroy(igxrt_scene* scene) {
     {
         DeviceGuard guard(scene->device);
         cudaDeviceSynchronize();
-        if (scene->pooled)
+        if (scene->pool)
             cudaFreeAsync(scene->d_mem, nullptr);
         else
             cudaFree(scene->d_mem);

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -13,6 +14,15 @@ namespace igxrt {
 // Ring of item tables used by igxrt_trace_batch.
 constexpr uint32_t kBatchSlots = 16;
 constexpr uint32_t kBatchSlotItems = 4096;
+
+// A device memory pool and what keeps it: its context, and every scene whose
+// memory it holds (the runtime does not survive a free into a destroyed
+// pool), so the last of them destroys it.
+struct MemoryPool {
+    cudaMemPool_t pool = nullptr;
+    int device = 0;
+    ~MemoryPool();
+};
 }  // namespace igxrt
 
 struct igxrt_context {
@@ -39,7 +49,7 @@ struct igxrt_context {
     // 300K-triangle frame).  Idle memory beyond kPoolKeep returns to the device
     // at the next synchronisation, the rest when the context and the last
     // scene are gone.  Null where the device has no pools.
-    cudaMemPool_t pool = nullptr;
+    std::shared_ptr<igxrt::MemoryPool> pool;
     // The device loads and stores pageable host memory through the host's
     // page tables (cudaDevAttrPageableMemoryAccessUsesHostPageTables).
     bool pageable_access = false;
@@ -49,7 +59,7 @@ struct igxrt_scene {
     int device = 0;
     igxrt_bvh_info info{};
     void* d_mem = nullptr;
-    bool pooled = false;  // d_mem is the context's pool's
+    std::shared_ptr<igxrt::MemoryPool> pool;  // d_mem's, if it came from one
     const void* nodes[IGXRT_LAYOUT_COUNT] = {nullptr, nullptr, nullptr};
     uint32_t node_count[IGXRT_LAYOUT_COUNT] = {0, 0, 0};
     const igxrt_prim_record* prims = nullptr;
