@@ -12,6 +12,7 @@
 #include "engine.h"
 #include "gbuffer.cuh"
 #include "grid.cuh"
+#include "leaf.cuh"
 #include "share.cuh"
 #include "traverse.cuh"
 
@@ -77,9 +78,10 @@ __device__ __forceinline__ void finish_ray(const KernelArgs& a, uint32_t i, cons
 // leaves every kernel's occupancy where it was.  The grid kernels run faster
 // without spills than with more warps: 56, 60, 64 and 72 registers take 2,553,
 // 2,586, 2,398 and 2,442 us on 4M incoherent rays over 2M triangles, and 461,
-// 452, 440 and 438 us on the 1M sphere's 1080p primaries.
+// 452, 440 and 438 us on the 1M sphere's 1080p primaries; the any-hit kernel
+// with the warp's leaf phase (leaf.cuh) spills below 70.
 constexpr int trace_kernel_regs(int layout, bool any, bool mixed) {
-    return layout == (int)kLayoutGrid    ? 64
+    return layout == (int)kLayoutGrid    ? (any && !mixed ? 72 : 64)
            : layout == IGXRT_LAYOUT_BVH2 ? (mixed && !any ? 64 : 56)
            : layout == IGXRT_LAYOUT_BVH4 ? (mixed && !any ? 72 : 64)
                                          : (any && !mixed ? 64 : 80);
@@ -109,6 +111,7 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
     if (!a.independent)
         asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr bool GRID = LAYOUT == (int)kLayoutGrid;
+    constexpr bool WARP_LEAVES = GRID && ANY && !MIXED;  // leaf.cuh
     extern __shared__ uint32_t smem[];
     TraversalStack st;
     st.sh = reinterpret_cast<uint2*>(smem) + threadIdx.x;
@@ -117,6 +120,7 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
     st.sp = 0;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lower = (1u << lane) - 1u;
+    uint2* list = reinterpret_cast<uint2*>(smem) + (size_t)a.sh_depth * blockDim.x + (threadIdx.x & ~31u);
     uint32_t pk_base = 0, pk_end = 0;  // warp-uniform window of claimed rays
     bool queue_done = false;           // warp-uniform
     bool alive = false, occluded_at_start = false;
@@ -200,15 +204,19 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
         // node phase: every lane of the warp takes part, the working lanes
         // descend (traverse.cuh: node_phase, which may end it early)
         bool overflow = false;
-        node_phase<LAYOUT, COUNT, MIXED>(a.nodes, working, wmask, a.phase_break, next, r, best, st, overflow, nf);
+        node_phase<LAYOUT, COUNT, MIXED>(a.nodes, working, wmask, a.phase_break, next, r, best, st, overflow, nf,
+                                            WARP_LEAVES && a.phase_break < 32u ? kLeafLanes : 33u);
+        bool leaf_occluded = false;
+        if constexpr (WARP_LEAVES)
+            any_leaf_phase(a.prims, working, lane, lower, list, next, r, best, st, leaf_occluded);
         if (working) {
             // a plane occluding the ray when it started decides it in this
             // first round; the flag must not outlive the ray (the lane may
             // next help another ray's traversal in the tail)
-            bool occluded = occluded_at_start;
+            bool occluded = occluded_at_start || leaf_occluded;
             occluded_at_start = false;
             // leaf phase
-            if (next < 0) {
+            if (!WARP_LEAVES && next < 0) {
                 occluded = GRID    ? process_grid_leaf<ANY, MIXED>(a.prims, next, r, best)
                            : MIXED ? process_leaf_mixed<ANY, COUNT>(a.prims, next, r, best, &pf)
                                    : process_leaf<ANY, COUNT>(a.prims, next, r, best, pf);
@@ -314,7 +322,8 @@ igxrt_status prepare_trace(igxrt_context* ctx, const TraceRequest& req, const ig
     l.fn = grid         ? select_grid_kernel(req.mode == 1, s->mixed, req.camera != nullptr)
            : req.camera ? select_camera_kernel(p.layout)
                         : select_kernel(p.layout, req.mode == 1, req.node_fetches != nullptr, s->mixed);
-    l.smem = (size_t)p.stack_depth * p.block_size * kStackEntryBytes;
+    l.smem = (size_t)p.stack_depth * p.block_size * kStackEntryBytes +
+             (grid && req.mode == 1 && !s->mixed ? p.block_size * kLeafEntryBytes : 0u);
     int per_sm = 0;
     cudaError_t e = allow_smem((const void*)l.fn, l.smem);
     if (e == cudaSuccess)

@@ -256,18 +256,20 @@ __device__ __forceinline__ int32_t visit_grid(const float4* __restrict__ nodes, 
 // working lanes waiting (at a leaf, or done), the phase ends and the
 // descending lanes resume in the warp's next round, after the leaves.  The
 // order in which each ray visits its nodes and records is the same for every
-// phase_break; phase_break 32 never ends the phase early.
+// phase_break; phase_break 32 never ends the phase early.  `enough` waiting
+// lanes end it too (33: no such number).
 template <int LAYOUT, bool COUNT, bool MIXED>
 __device__ __forceinline__ void node_phase(const float4* __restrict__ nodes, bool working, uint32_t wmask,
                                            uint32_t phase_break, int32_t& next, const RayState& r,
                                            const BestHit& best, TraversalStack& st, bool& overflow,
-                                           uint32_t& nf) {
+                                           uint32_t& nf, uint32_t enough = 33u) {
     for (;;) {
         const bool down = working && next >= 0 && next != kRefDone;
         const uint32_t dm = __ballot_sync(0xffffffffu, down);
         if (dm == 0)
             break;
-        if ((uint32_t)__popc(dm) * phase_break <= (uint32_t)__popc(wmask & ~dm))
+        const uint32_t waiting = (uint32_t)__popc(wmask & ~dm);
+        if ((uint32_t)__popc(dm) * phase_break <= waiting || waiting >= enough)
             break;
         if (down) {
             if constexpr (LAYOUT == (int)kLayoutGrid)
