@@ -75,11 +75,21 @@ struct BatchLane {
     }
 };
 
+// Register budget: the grid kernels keep 28 warps per SM at 72 registers; 64
+// spill and 80 hold 24 warps (a batch of 24 scenes: 340, 307 and 326 us at 64,
+// 72 and 80).  The others are held at what they need.
+constexpr int batch_kernel_regs(int layout, bool mixed) {
+    return layout == (int)kLayoutGrid     ? 72
+           : layout == IGXRT_LAYOUT_BVH2 ? (mixed ? 80 : 64)
+           : layout == IGXRT_LAYOUT_BVH4 ? 80
+                                         : (mixed ? 104 : 80);
+}
+
 // MIXED: items may hold spheres, cubes and planes (typed leaves, planes tested
 // when a ray starts, priority-coded best hit); triangle-only items trace the
 // same in it.
 template <int LAYOUT, bool MIXED>
-__global__ void __launch_bounds__(256) batch_kernel(BatchArgs a) {
+__global__ void __maxnreg__(batch_kernel_regs(LAYOUT, MIXED)) batch_kernel(BatchArgs a) {
     if (a.times && threadIdx.x == 0)
         atomicMin(a.times, global_ns());
     constexpr bool GRID = LAYOUT == (int)kLayoutGrid;

