@@ -47,13 +47,15 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // A finished ray's record: occluded word (any hit) or hit (closest).  Mixed
 // scenes keep a priority code in best.prim (traverse.cuh), decoded here.
 template <bool MIXED>
-__device__ __forceinline__ void write_result(void* out, uint32_t mode, uint32_t ray, const RayState& r,
-                                             const BestHit& best, bool occluded) {
+__device__ __forceinline__ void write_result(void* out, const float4* __restrict__ prims, uint32_t mode,
+                                             uint32_t ray, const RayState& r, BestHit& best, bool occluded) {
     if (mode) {
         __stcs(static_cast<uint32_t*>(out) + ray, occluded ? 1u : 0u);
     } else {
         const bool hit = MIXED ? (best.t < r.tmax_eff || best.prim < kPrioNone) : best.t < r.tmax_eff;
         const uint32_t prim = MIXED ? id_of_prio(best.prim) : best.prim;
+        if (MIXED)
+            finish_uv(prims, r, best);
         const float4 h = hit ? make_float4(best.t, best.u, best.v, __uint_as_float(prim))
                              : make_float4(IGXRT_NO_HIT, 0.f, 0.f, __uint_as_float(IGXRT_NO_RAY_HIT));
         __stcs(static_cast<float4*>(out) + ray, h);
@@ -120,7 +122,7 @@ __global__ void __maxnreg__(batch_kernel_regs(LAYOUT, MIXED)) batch_kernel(Batch
         if (queue_done && __ballot_sync(0xffffffffu, !alive || (link & (kLinkWait | kLinkMerge))) != 0) {
             BatchLane lane_item{nodes, prims, out, mode};
             share_tail<kSharePerLane>(lane, lower, link, alive, ray, r, best, st, next, lane_item,
-                                      [&](bool occ) { write_result<MIXED>(out, mode, ray, r, best, occ); },
+                                      [&](bool occ) { write_result<MIXED>(out, prims, mode, ray, r, best, occ); },
                                       MIXED ? kPrioNone : 0u);
         }
         const uint32_t idle = __ballot_sync(0xffffffffu, !alive);
@@ -223,7 +225,7 @@ __global__ void __maxnreg__(batch_kernel_regs(LAYOUT, MIXED)) batch_kernel(Batch
                     // share_tail writes the ray once no helper of it remains
                     link |= ((link & 31u) == lane ? kLinkWait : kLinkMerge) | (occluded ? kLinkOcc : 0u);
                 } else {
-                    write_result<MIXED>(out, mode, ray, r, best, occluded);
+                    write_result<MIXED>(out, prims, mode, ray, r, best, occluded);
                     alive = false;
                 }
             }

@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(256) gbuffer_kernel(GbufferArgs a) {
             atomicOr(a.status, gave_up);
         if (!inside)
             continue;
+        if (MIXED)
+            finish_uv(a.prims, r, best);
         const size_t px = (size_t)y * g.cam.width + x;
         // raygen.comp:39-44: a miss is hitT == noHit
         const bool hit = best.t < IGXRT_NO_HIT;

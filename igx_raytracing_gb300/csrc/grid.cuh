@@ -159,11 +159,11 @@ __device__ __forceinline__ int32_t visit_grid(const float4* __restrict__ nodes, 
 template <bool ANY, bool MIXED>
 __device__ __forceinline__ bool process_grid_leaf(const float4* __restrict__ prims, int32_t ref, const RayState& r,
                                                   BestHit& best) {
-    const uint32_t first = ((uint32_t)ref & ~kGridLeaf) >> 4;
-    const float4* p = prims + 3 * (size_t)first;
-    for (int32_t more = ref & 15;; --more, p += 3) {
+    uint32_t i = ((uint32_t)ref & ~kGridLeaf) >> 4;
+    const float4* p = prims + 3 * (size_t)i;
+    for (int32_t more = ref & 15;; --more, ++i, p += 3) {
         const float4 v0 = __ldg(p), v1 = __ldg(p + 1), v2 = __ldg(p + 2);
-        if ((MIXED ? test_record_mixed<ANY>(v0, v1, v2, 0, r, best) : test_record<ANY>(v0, v1, v2, r, best)) && ANY)
+        if ((MIXED ? test_record_mixed<ANY>(v0, v1, v2, i, r, best) : test_record<ANY>(v0, v1, v2, r, best)) && ANY)
             return true;
         if (more == 0)
             return false;

@@ -56,13 +56,15 @@ struct KernelArgs {
 
 template <bool ANY, bool COUNT, bool MIXED>
 __device__ __forceinline__ void finish_ray(const KernelArgs& a, uint32_t i, const RayState& r,
-                                           const BestHit& best, bool occluded, uint32_t nf,
+                                           BestHit& best, bool occluded, uint32_t nf,
                                            uint32_t pf) {
     if (ANY) {
         __stcs(a.occluded + i, occluded ? 1u : 0u);
     } else {
         const bool hit = MIXED ? (best.t < r.tmax_eff || best.prim < kPrioNone) : best.t < r.tmax_eff;
         const uint32_t prim = MIXED ? id_of_prio(best.prim) : best.prim;
+        if (MIXED)
+            finish_uv(a.prims, r, best);
         const float4 h = hit ? make_float4(best.t, best.u, best.v, __uint_as_float(prim))
                              : make_float4(IGXRT_NO_HIT, 0.f, 0.f, __uint_as_float(IGXRT_NO_RAY_HIT));
         __stcs(reinterpret_cast<float4*>(a.hits) + i, h);
@@ -71,6 +73,32 @@ __device__ __forceinline__ void finish_ray(const KernelArgs& a, uint32_t i, cons
         a.node_fetches[i] = nf;
         a.prim_fetches[i] = pf;
     }
+}
+
+// Sphere hits whose uv is still to come (finish_uv), collected by a warp of a
+// mixed scene's closest-hit kernel until there is one for every lane: the uv
+// takes binary64 asin and atan, and with a lane or two of a warp at a time
+// they kept that pipe half busy on 1M rays of which 15% hit a sphere (664 us;
+// 615 in batches; 602 with no uv at all).  In shared memory, per warp: the
+// number of entries, then {ray, record, t} each; fewer than 32 are left after
+// a flush and a round adds at most one per lane.
+constexpr uint32_t kUvEntries = 64, kUvWords = 4 + 3 * kUvEntries;
+
+__device__ __forceinline__ void flush_uv(const KernelArgs& a, uint32_t* batch, uint32_t take, uint32_t lane) {
+    const uint32_t base = batch[0] - take;
+    if (lane < take) {
+        const uint32_t* e = batch + 4 + 3 * (base + lane);
+        const RayState r = load_ray(a.rays, e[0], 0u);
+        const float4 c = __ldg(a.prims + 3 * (size_t)e[1]);
+        const float t = __uint_as_float(e[2]);
+        float u, v;
+        sphere_uv(r, c.x, c.y, c.z, t, u, v);
+        __stcs(reinterpret_cast<float4*>(a.hits) + e[0], make_float4(t, u, v, c.w));  // c.w: the object
+    }
+    __syncwarp();
+    if (lane == 0)
+        batch[0] = base;
+    __syncwarp();
 }
 
 // Register budget per instantiation: what each reached before the tail
@@ -120,7 +148,15 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
     st.sp = 0;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lower = (1u << lane) - 1u;
+    constexpr bool UV_BATCH = MIXED && !ANY && !COUNT;
+    // after the stacks: the warp's leaf list, or its pending sphere hits
     uint2* list = reinterpret_cast<uint2*>(smem) + (size_t)a.sh_depth * blockDim.x + (threadIdx.x & ~31u);
+    uint32_t* uv = smem + 2 * (size_t)a.sh_depth * blockDim.x + (threadIdx.x >> 5) * kUvWords;
+    if (UV_BATCH) {
+        if (lane == 0)
+            uv[0] = 0;
+        __syncwarp();
+    }
     uint32_t pk_base = 0, pk_end = 0;  // warp-uniform window of claimed rays
     bool queue_done = false;           // warp-uniform
     bool alive = false, occluded_at_start = false;
@@ -133,14 +169,28 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
     // the single-lane order their fetch counts describe
     constexpr bool STEAL = !COUNT;
     uint32_t link = lane;
+    const auto write_ray = [&](bool occluded) {
+        if (UV_BATCH && __float_as_uint(best.v) == kUvPending) {
+            uint32_t* e = uv + 4 + 3 * atomicAdd(uv, 1u);
+            e[0] = ray;
+            e[1] = __float_as_uint(best.u);
+            e[2] = __float_as_uint(best.t);
+        } else {
+            finish_ray<ANY, COUNT, MIXED>(a, ray, r, best, occluded, nf, pf);
+        }
+    };
     for (;;) {
+        if (UV_BATCH) {
+            __syncwarp();
+            if (uv[0] >= 32u)
+                flush_uv(a, uv, 32u, lane);
+        }
         if (STEAL && queue_done &&
             __ballot_sync(0xffffffffu, !alive || (link & (kLinkWait | kLinkMerge))) != 0) {
             NoLaneExtra none;
             share_tail<ANY ? kShareAny : kShareClosest>(
                 lane, lower, link, alive, ray, r, best, st, next, none,
-                [&](bool occ) { finish_ray<ANY, false, MIXED>(a, ray, r, best, occ, 0, 0); },
-                MIXED ? kPrioNone : 0u);
+                write_ray, MIXED ? kPrioNone : 0u);
         }
         const uint32_t idle = __ballot_sync(0xffffffffu, !alive);
         const uint32_t nidle = __popc(idle);
@@ -230,11 +280,16 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
                     // share_tail writes the ray once no helper of it remains
                     link |= ((link & 31u) == lane ? kLinkWait : kLinkMerge) | (occluded ? kLinkOcc : 0u);
                 } else {
-                    finish_ray<ANY, COUNT, MIXED>(a, ray, r, best, occluded, nf, pf);
+                    write_ray(occluded);
                     alive = false;
                 }
             }
         }
+    }
+    if (UV_BATCH) {
+        __syncwarp();
+        while (uv[0])
+            flush_uv(a, uv, min(uv[0], 32u), lane);
     }
     if (a.exit_count && lane == 0) {
         // every warp's queue claims come before its exit count
@@ -323,7 +378,8 @@ igxrt_status prepare_trace(igxrt_context* ctx, const TraceRequest& req, const ig
            : req.camera ? select_camera_kernel(p.layout)
                         : select_kernel(p.layout, req.mode == 1, req.node_fetches != nullptr, s->mixed);
     l.smem = (size_t)p.stack_depth * p.block_size * kStackEntryBytes +
-             (grid && req.mode == 1 && !s->mixed ? p.block_size * kLeafEntryBytes : 0u);
+             (s->mixed ? (req.mode == 0 ? p.block_size / 32 * kUvWords * 4u : 0u)
+                       : (grid && req.mode == 1 ? p.block_size * kLeafEntryBytes : 0u));
     int per_sm = 0;
     cudaError_t e = allow_smem((const void*)l.fn, l.smem);
     if (e == cudaSuccess)

@@ -598,9 +598,10 @@ __device__ __forceinline__ void sphere_uv(const RayState& r, float cx, float cy,
 }
 
 // rayIntersectCube (primitive.glsl:286-333) with the ray's raw 1/dir.
-// Returns whether [tmin, tmax] is a valid interval reaching tmin_ray.
+// Returns whether [tmin, tmax] is a valid interval reaching tmin_ray, and the
+// axis the ray enters on (cube_uv).
 __device__ __forceinline__ bool cube_hit(const RayState& r, const float4& s, const float4& e, float& tmin,
-                                         float& u, float& v) {
+                                         int& axis) {
     const float rx = __frcp_rn(r.dx), ry = __frcp_rn(r.dy), rz = __frcp_rn(r.dz);
     const float sx = __fmul_rn(__fsub_rn(s.x, r.ox), rx), sy = __fmul_rn(__fsub_rn(s.y, r.oy), ry),
                 sz = __fmul_rn(__fsub_rn(s.z, r.oz), rz);
@@ -610,23 +611,20 @@ __device__ __forceinline__ bool cube_hit(const RayState& r, const float4& s, con
     const float max_ = gmax(sx, ex), may = gmax(sy, ey), maz = gmax(sz, ez);
     tmin = gmax(gmax(mix, miy), miz);
     const float tmax = gmin(gmin(max_, may), maz);
-    if (tmax < r.tmin || tmin > tmax)
-        return false;
+    axis = tmin == mix ? 0 : (tmin == miy ? 1 : 2);
+    return !(tmax < r.tmin || tmin > tmax);
+}
+
+// The cube's uv at its entry distance; the three divisions are left to the
+// candidates that become the best hit.
+__device__ __forceinline__ void cube_uv(const RayState& r, const float4& s, const float4& e, float tmin, int axis,
+                                        float& u, float& v) {
     // pos = (dir * tmin + pos) - start; pos /= end
     const float px = __fdiv_rn(__fsub_rn(__fadd_rn(__fmul_rn(r.dx, tmin), r.ox), s.x), e.x);
     const float py = __fdiv_rn(__fsub_rn(__fadd_rn(__fmul_rn(r.dy, tmin), r.oy), s.y), e.y);
     const float pz = __fdiv_rn(__fsub_rn(__fadd_rn(__fmul_rn(r.dz, tmin), r.oz), s.z), e.z);
-    if (tmin == mix) {
-        u = py;
-        v = pz;
-    } else if (tmin == miy) {
-        u = px;
-        v = pz;
-    } else {
-        u = px;
-        v = py;
-    }
-    return true;
+    u = axis == 0 ? py : px;
+    v = axis == 2 ? py : pz;
 }
 
 // rayIntersectPlane (primitive.glsl:212-237): hitT, and the uv on request.
@@ -650,6 +648,17 @@ __device__ __forceinline__ void plane_uv(const RayState& r, const float4& pl, fl
     const float zz = __fsub_rn(__fmul_rn(pl.x, 0.0f), __fmul_rn(1.0f, pl.y));
     u = dot3f(ox, oy, oz, xx, xy, xz);
     v = dot3f(ox, oy, oz, zx, zy, zz);
+}
+
+// A sphere that becomes the best hit leaves its record index in u and this
+// word (a NaN no arithmetic yields) in v; finish_uv evaluates the uv, whose
+// asin and atan are binary64, once the ray's hit is known.
+constexpr uint32_t kUvPending = 0xffffffffu;
+__device__ __forceinline__ void finish_uv(const float4* __restrict__ prims, const RayState& r, BestHit& best) {
+    if (__float_as_uint(best.v) != kUvPending)
+        return;
+    const float4 c = __ldg(prims + 3 * (size_t)__float_as_uint(best.u));
+    sphere_uv(r, c.x, c.y, c.z, best.t, best.u, best.v);
 }
 
 // Record `i` of a mixed scene against the ray.  Returns true when an any-hit
@@ -683,20 +692,21 @@ __device__ __forceinline__ bool test_record_mixed(const float4& v0, const float4
             return t < r.tmax_eff;
         if (!better(t, prio_other(id), best))
             return false;
-        sphere_uv(r, v0.x, v0.y, v0.z, t, best.u, best.v);
+        best.u = __uint_as_float(i);  // finish_uv
+        best.v = __uint_as_float(kUvPending);
         best.t = t;
         best.prim = prio_other(id);
     } else {
-        float t, u, v;
-        if (!cube_hit(r, v0, v1, t, u, v))
+        float t;
+        int axis;
+        if (!cube_hit(r, v0, v1, t, axis))
             return false;
         if (ANY)
             return t < r.tmax_eff;
         if (!better(t, prio_cube(id), best))
             return false;
+        cube_uv(r, v0, v1, t, axis, best.u, best.v);
         best.t = t;
-        best.u = u;
-        best.v = v;
         best.prim = prio_cube(id);
     }
     best.tcull = cull_limit(best.t);
