@@ -65,6 +65,7 @@ __device__ __forceinline__ void write_result(void* out, const float4* __restrict
 // A lane's item (scene arrays, output, query mode), which a helper in the
 // tail copies from the lane whose ray it helps (share.cuh).
 struct BatchLane {
+    static constexpr bool kRayInShared = false;
     const float4*& nodes;
     const float4*& prims;
     void*& out;

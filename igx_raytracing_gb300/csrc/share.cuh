@@ -30,13 +30,14 @@ constexpr int kShareClosest = 0, kShareAny = 1, kSharePerLane = 2;
 
 // No per-lane state beyond the ray (the plain trace kernels).
 struct NoLaneExtra {
+    static constexpr bool kRayInShared = false;
     __device__ __forceinline__ void take(uint32_t) {}
 };
 
 // One round of tail work sharing, run by the whole warp between traversal
 // phases.  `extra` holds lane state a helper must copy from its victim
 // (take(src) reads it from lane src; lanes that take nothing read their
-// own); `finish(occluded)` writes the lane's ray; `no_hit` is the value of
+// own), with kRayInShared the ray's origin, direction and tmin among it; `finish(occluded)` writes the lane's ray; `no_hit` is the value of
 // BestHit.prim before a first hit (0, or the priority code of mixed
 // scenes, whose merges then compare (t, priority) like their leaves do).
 template <int MODE, class Extra, class Finish>
@@ -120,19 +121,21 @@ __device__ __forceinline__ void share_tail(uint32_t lane, uint32_t lower, uint32
     const uint32_t vray = __shfl_sync(FULL, ray, src), vlink = __shfl_sync(FULL, link, src);
     const float vtc = __shfl_sync(FULL, best.tcull, src);
     // the victim's ray, read in place: a lane that is no thief reads its own
-    r.ox = __shfl_sync(FULL, r.ox, src);
-    r.oy = __shfl_sync(FULL, r.oy, src);
-    r.oz = __shfl_sync(FULL, r.oz, src);
-    r.dx = __shfl_sync(FULL, r.dx, src);
-    r.dy = __shfl_sync(FULL, r.dy, src);
-    r.dz = __shfl_sync(FULL, r.dz, src);
+    if constexpr (!Extra::kRayInShared) {
+        r.ox = __shfl_sync(FULL, r.ox, src);
+        r.oy = __shfl_sync(FULL, r.oy, src);
+        r.oz = __shfl_sync(FULL, r.oz, src);
+        r.dx = __shfl_sync(FULL, r.dx, src);
+        r.dy = __shfl_sync(FULL, r.dy, src);
+        r.dz = __shfl_sync(FULL, r.dz, src);
+        r.tmin = __shfl_sync(FULL, r.tmin, src);
+    }
     r.ix = __shfl_sync(FULL, r.ix, src);
     r.iy = __shfl_sync(FULL, r.iy, src);
     r.iz = __shfl_sync(FULL, r.iz, src);
     r.oix = __shfl_sync(FULL, r.oix, src);
     r.oiy = __shfl_sync(FULL, r.oiy, src);
     r.oiz = __shfl_sync(FULL, r.oiz, src);
-    r.tmin = __shfl_sync(FULL, r.tmin, src);
     r.tmin_box = __shfl_sync(FULL, r.tmin_box, src);
     r.tmax_eff = __shfl_sync(FULL, r.tmax_eff, src);
     r.prev = __shfl_sync(FULL, r.prev, src);

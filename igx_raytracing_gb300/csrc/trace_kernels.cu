@@ -8,6 +8,7 @@
 // 128-bit read-only loads; hit records are written with streaming stores so
 // they do not displace BVH lines from L2.
 #include <algorithm>
+#include <type_traits>
 
 #include "engine.h"
 #include "gbuffer.cuh"
@@ -106,8 +107,8 @@ __device__ __forceinline__ void flush_uv(const KernelArgs& a, uint32_t* batch, u
 // leaves every kernel's occupancy where it was.  The grid kernels run faster
 // without spills than with more warps: 56, 60, 64 and 72 registers take 2,553,
 // 2,586, 2,398 and 2,442 us on 4M incoherent rays over 2M triangles, and 461,
-// 452, 440 and 438 us on the 1M sphere's 1080p primaries; the any-hit kernel
-// with the warp's leaf phase (leaf.cuh) spills below 70.
+// 452, 440 and 438 us on the 1M sphere's 1080p primaries.  The any-hit kernel
+// gains from 72 (1M occlusion rays 356 us, 364 at 64).
 constexpr int trace_kernel_regs(int layout, bool any, bool mixed) {
     return layout == (int)kLayoutGrid    ? (any && !mixed ? 72 : 64)
            : layout == IGXRT_LAYOUT_BVH2 ? (mixed && !any ? 64 : 56)
@@ -139,7 +140,7 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
     if (!a.independent)
         asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr bool GRID = LAYOUT == (int)kLayoutGrid;
-    constexpr bool WARP_LEAVES = GRID && ANY && !MIXED;  // leaf.cuh
+    constexpr bool WARP_LEAVES = GRID && !MIXED;  // leaf.cuh
     extern __shared__ uint32_t smem[];
     TraversalStack st;
     st.sh = reinterpret_cast<uint2*>(smem) + threadIdx.x;
@@ -149,9 +150,10 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lower = (1u << lane) - 1u;
     constexpr bool UV_BATCH = MIXED && !ANY && !COUNT;
-    // after the stacks: the warp's leaf list, or its pending sphere hits
-    uint2* list = reinterpret_cast<uint2*>(smem) + (size_t)a.sh_depth * blockDim.x + (threadIdx.x & ~31u);
-    uint32_t* uv = smem + 2 * (size_t)a.sh_depth * blockDim.x + (threadIdx.x >> 5) * kUvWords;
+    // after the stacks: the warp's leaf phase, or its pending sphere hits
+    uint32_t* after = smem + 2 * (size_t)a.sh_depth * blockDim.x;
+    WarpLeaves& leaves = *reinterpret_cast<WarpLeaves*>(after + (threadIdx.x >> 5) * (leaf_bytes(ANY) / 4u));
+    uint32_t* uv = after + (threadIdx.x >> 5) * kUvWords;
     if (UV_BATCH) {
         if (lane == 0)
             uv[0] = 0;
@@ -187,9 +189,11 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
         }
         if (STEAL && queue_done &&
             __ballot_sync(0xffffffffu, !alive || (link & (kLinkWait | kLinkMerge))) != 0) {
-            NoLaneExtra none;
+            std::conditional_t<WARP_LEAVES, SharedRay, NoLaneExtra> extra;
+            if constexpr (WARP_LEAVES)
+                extra = {&leaves, lane};
             share_tail<ANY ? kShareAny : kShareClosest>(
-                lane, lower, link, alive, ray, r, best, st, next, none,
+                lane, lower, link, alive, ray, r, best, st, next, extra,
                 write_ray, MIXED ? kPrioNone : 0u);
         }
         const uint32_t idle = __ballot_sync(0xffffffffu, !alive);
@@ -226,6 +230,8 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
                     best.t = r.tmax_eff;
                     best.u = 0.f;
                     best.v = 0.f;
+                    if (WARP_LEAVES)
+                        leaves.put(lane, r);
                     if (GRID)
                         to_grid(r, a.grid);
                     // "prim < best.prim" cannot hold before a first hit
@@ -258,7 +264,7 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
                                             WARP_LEAVES && a.phase_break < 32u ? kLeafLanes : 33u);
         bool leaf_occluded = false;
         if constexpr (WARP_LEAVES)
-            any_leaf_phase(a.prims, working, lane, lower, list, next, r, best, st, leaf_occluded);
+            warp_leaf_phase<ANY>(a.prims, working, lane, lower, leaves, next, r.prev, best, st, leaf_occluded);
         if (working) {
             // a plane occluding the ray when it started decides it in this
             // first round; the flag must not outlive the ray (the lane may
@@ -378,8 +384,8 @@ igxrt_status prepare_trace(igxrt_context* ctx, const TraceRequest& req, const ig
            : req.camera ? select_camera_kernel(p.layout)
                         : select_kernel(p.layout, req.mode == 1, req.node_fetches != nullptr, s->mixed);
     l.smem = (size_t)p.stack_depth * p.block_size * kStackEntryBytes +
-             (s->mixed ? (req.mode == 0 ? p.block_size / 32 * kUvWords * 4u : 0u)
-                       : (grid && req.mode == 1 ? p.block_size * kLeafEntryBytes : 0u));
+             p.block_size / 32 * (s->mixed ? (req.mode == 0 ? kUvWords * 4u : 0u)
+                                           : (grid ? leaf_bytes(req.mode == 1) : 0u));
     int per_sm = 0;
     cudaError_t e = allow_smem((const void*)l.fn, l.smem);
     if (e == cudaSuccess)

@@ -1,4 +1,4 @@
-"""Any-hit leaves tested by the whole warp (csrc/leaf.cuh): the occluded words
+"""Leaves tested by the whole warp (csrc/leaf.cuh): hits and occluded words
 against the brute-force oracle, bit for bit, with leaves from one record to
 the most a leaf holds (16), so that a phase's pairs end before, on and after
 its turns of 32; with rays that stop inside the scene, an excluded object,
@@ -27,12 +27,18 @@ def test_leaf_lengths(ctx, leaf, phase_break):
     want, flags = pyoracle.trace_occlusion(tris, rays, prev)
     ok = flags == 0
     assert 0.05 < want[ok].mean() < 0.95
+    closest, flags = pyoracle.trace_geometry(tris, rays, prev)
+    near = flags == 0
     saved = ctx.launch_params
     try:
         ctx.set_launch_params(layout=0, phase_break=phase_break)
         for n in (1, 5, 31, 32, 33, 777, 6000):
             got = scene.trace_occlusion(rays[:n], prev[:n])
             assert np.array_equal(got[ok[:n]], want[:n][ok[:n]]), (leaf, n)
+            hits = scene.trace_geometry(rays[:n], prev[:n])
+            for f in ("prim", "t", "u", "v"):
+                a, b = (x[f][:n][near[:n]].view(np.uint32) for x in (hits, closest))
+                assert np.array_equal(a, b), (leaf, n, f)
     finally:
         ctx.set_launch_params(**saved)
     scene.close()
