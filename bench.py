@@ -1450,9 +1450,10 @@ def run_dynamic_bench(args, rank: int, world: int, local_rank: int):
     nf, pf = ctx.count_fetches(scene, rays, None, mode=0, layout=layout)
     n = len(rays)
     b = algorithmic_bytes(nf, pf, 0, False, layout)
-    # a frame: the refit's scan, records, nodes and BVH8 passes, then the trace
+    # a frame: the refit's scan, records, nodes, BVH8 and grid passes, then the trace
     si = scene.info
-    refit_launches = 2 + (si["bvh2_nodes"] + si["bvh4_nodes"] > 0) + (si["bvh8_nodes"] > 0) + 1
+    refit_launches = (2 + (si["bvh2_nodes"] + si["bvh4_nodes"] > 0) + (si["bvh8_nodes"] > 0)
+                      + (si["bvh4_nodes"] > 0) + 1)
     cfg = {"workload": "dynamic_sphere_1m_refit_1080p_primary", "triangles": len(tris),
            "rays_per_step": n, "layout": LAYOUT_NAMES[layout], "launch": ctx.launch_params,
            "frames": len(frames), "host_sah_build_s": round(host_build_s, 3),

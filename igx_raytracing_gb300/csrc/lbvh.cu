@@ -47,6 +47,11 @@ constexpr int kMaxLevels = 64;     // > key bits: no path is longer
 // about log4 of its leaves, 10 at 300K objects; an empty level costs 1.2 us,
 // and one block takes whatever levels are left (bvh4_rest_kernel).
 constexpr int kWideLevels = 20;
+// Largest scene whose BVH4 levels all run in that block, where a level costs no
+// launch but has one SM: whole builds of 4,000 / 8,000 / 16,000 / 32,000 /
+// 64,000 triangles take 247 / 248 / 256 / 263 / 280 us with launched levels
+// and 204 / 218 / 242 / 279 / 390 in the block.
+constexpr uint32_t kOneBlock = 16384;
 constexpr int kStateWords = kWordLevels + kMaxLevels + 1;
 constexpr uint32_t kDefaultLeaf = 4;
 
@@ -101,6 +106,8 @@ __global__ void morton_kernel(BuildArgs a, uint64_t* keys) {
     const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= a.n)
         return;
+    if (id + 1 < a.n)
+        a.arrive[id] = 0;  // the climb's counters
     const Box b = object_box<false>(a.obj, id);
     uint32_t code = 0;
     for (int k = 0; k < 3; ++k) {
@@ -230,6 +237,10 @@ __global__ void __launch_bounds__(256) emit2_kernel(BuildArgs a) {
         if (i == root) {
             a.parents2[0] = kNoParent;
             a.state[kWordNodes2] = a.map[a.n - 2] + a.live[a.n - 2];
+            // the first BVH4 level: the root
+            a.frontier[0][0] = make_uint2(0, 0);
+            a.state[kWordLevels] = 1;
+            a.parents4[0] = kNoParent;
         }
     }
     __shared__ double block_sah[8];
@@ -287,12 +298,6 @@ __global__ void emit_single_leaf_kernel(BuildArgs a) {
     a.state[kWordLeaves] = 1;
     a.state[kWordDepth] = 1;
     *reinterpret_cast<double*>(a.state + kWordSah) = (double)a.n;
-}
-
-__global__ void bvh4_root_kernel(BuildArgs a) {
-    a.frontier[0][0] = make_uint2(0, 0);
-    a.state[kWordLevels] = a.state[kWordMalformed] ? 0u : 1u;
-    a.parents4[0] = kNoParent;
 }
 
 // One BVH4 level: each frontier BVH2 node becomes a BVH4 node whose slots are
@@ -452,14 +457,38 @@ __global__ void __launch_bounds__(256) emit4_level_kernel(BuildArgs a, int level
     emit4_level(a, level, warp * 32u + (threadIdx.x & 31u), gridDim.x * blockDim.x);
 }
 
-// The levels after them, one block: empty but for deep trees, whose last
-// levels are mostly narrow.
-__global__ void __launch_bounds__(1024) bvh4_rest_kernel(BuildArgs a) {
+// The levels from `first` on, one block: empty but for deep trees, whose last
+// levels are mostly narrow, and all levels of small scenes, where a level in
+// the block costs 3 us and a launch 5.5 (kOneBlock).
+__global__ void __launch_bounds__(1024) bvh4_rest_kernel(BuildArgs a, int first) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int level = kWideLevels; level < kMaxLevels; ++level) {
+    for (int level = first; level < kMaxLevels; ++level) {
         if (emit4_level(a, level, threadIdx.x, blockDim.x) == 0)
             return;
         __syncthreads();
+    }
+}
+
+// The finished arrays, from the build's scratch (and the caller's triangles and
+// planes) into the scene: up to kCopies segments of whole 4-byte words in one
+// launch, 16 bytes at a time where both ends are aligned.  Seven copies in a
+// row took a launch gap each.
+constexpr int kCopies = 7;
+struct CopyList {
+    const uint32_t* src[kCopies];
+    uint32_t* dst[kCopies];
+    uint64_t words[kCopies];
+};
+
+__global__ void __launch_bounds__(256) copy_kernel(CopyList c) {
+    const uint64_t first = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = gridDim.x * (uint64_t)blockDim.x;
+    for (int k = 0; k < kCopies; ++k) {
+        const bool wide = (((uintptr_t)c.src[k] | (uintptr_t)c.dst[k]) & 15u) == 0;
+        const uint64_t quads = wide ? c.words[k] / 4 : 0;
+        for (uint64_t i = first; i < quads; i += step)
+            reinterpret_cast<uint4*>(c.dst[k])[i] = __ldcs(reinterpret_cast<const uint4*>(c.src[k]) + i);
+        for (uint64_t i = 4 * quads + first; i < c.words[k]; i += step)
+            c.dst[k][i] = __ldcs(c.src[k] + i);
     }
 }
 
@@ -560,8 +589,6 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
     const uint32_t threads = 256;
     auto blocks = [threads](size_t count) { return (uint32_t)std::max<size_t>((count + threads - 1) / threads, 1); };
     e = cudaMemsetAsync(a.state, 0, kStateWords * 4, s);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(a.arrive, 0, ni * 4, s);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "build state reset");
     const uint32_t scan_grid = std::min<uint32_t>(blocks(std::max<size_t>({(size_t)n, 4 * (size_t)a.obj.np, 1})),
@@ -587,7 +614,6 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
         if (e != cudaSuccess)
             return cuda_fail(ctx, e, "node compaction");
         emit2_kernel<<<std::min<uint32_t>(blocks(n - 1), (uint32_t)std::max(ctx->sm_count, 1) * 8), threads, 0, s>>>(a);
-        bvh4_root_kernel<<<1, 1, 0, s>>>(a);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((uint32_t)std::max(ctx->sm_count, 1) * 4);
         cfg.blockDim = dim3(threads);
@@ -597,12 +623,13 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        for (int level = 0; level < kWideLevels && e == cudaSuccess; ++level)
+        const int wide = n <= kOneBlock ? 0 : kWideLevels;
+        for (int level = 0; level < wide && e == cudaSuccess; ++level)
             e = cudaLaunchKernelEx(&cfg, emit4_level_kernel, a, level);
         cfg.gridDim = dim3(1);
         cfg.blockDim = dim3(1024);
         if (e == cudaSuccess)
-            e = cudaLaunchKernelEx(&cfg, bvh4_rest_kernel, a);
+            e = cudaLaunchKernelEx(&cfg, bvh4_rest_kernel, a, wide);
         if (e != cudaSuccess)
             return cuda_fail(ctx, e, "BVH4 level launch");
     }
@@ -662,9 +689,12 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
     igxrt_scene* scene = nullptr;
     if ((st = allocate_scene(ctx, info, n2, n4, 0, scene, true, s)) != IGXRT_OK)
         return st;
+    CopyList copies{};
+    int parts = 0;
     auto copy = [&](const void* dst, const void* src, size_t bytes) {
-        if (e == cudaSuccess && bytes)
-            e = cudaMemcpyAsync(const_cast<void*>(dst), src, bytes, cudaMemcpyDeviceToDevice, s);
+        copies.src[parts] = static_cast<const uint32_t*>(src);
+        copies.dst[parts] = static_cast<uint32_t*>(const_cast<void*>(dst));
+        copies.words[parts++] = bytes / 4;
     };
     copy(scene->nodes[IGXRT_LAYOUT_BVH2], a.nodes2, sizeof(igxrt_bvh2_node) * (size_t)n2);
     copy(scene->nodes[IGXRT_LAYOUT_BVH4], a.nodes4, sizeof(igxrt_bvh4_node) * (size_t)n4);
@@ -673,6 +703,10 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
     copy(scene->prims, a.prims, sizeof(igxrt_prim_record) * (size_t)n);
     copy(scene->tris, a.obj.tris, sizeof(igxrt_triangle) * (size_t)a.obj.nt);
     copy(scene->planes, a.obj.planes, 16 * (size_t)a.obj.np);
+    copy_kernel<<<std::min<uint32_t>(blocks(std::max<size_t>(3 * (size_t)n, 1)), (uint32_t)std::max(ctx->sm_count, 1) * 8),
+                  threads, 0, s>>>(copies);
+    if (e == cudaSuccess)
+        e = cudaGetLastError();
     if (e == cudaSuccess)
         e = cudaMemsetAsync(scene->refit_words, 0, kRefitStateWords * sizeof(uint32_t), s);
     if (e == cudaSuccess)
