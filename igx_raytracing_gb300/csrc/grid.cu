@@ -26,6 +26,11 @@ __device__ GridAxis grid_axis(float lo, float hi) {
             break;
         g.scale = __fmul_ru(g.scale, 1.000001f);
     }
+    // a range near the end of the floats: launches go to the exact nodes
+    // (grid_usable), and a captured batch that kept these finds the axis out
+    // of its box tests (to_grid) instead of boxes at infinity
+    if (!isfinite(g.scale) || !isfinite(g.origin))
+        g.scale = __int_as_float(0x7fffffff);
     g.inv = 1.f / g.scale;
     return g;
 }
