@@ -97,10 +97,9 @@ cudaError_t pool_alloc(igxrt_context* ctx, void** ptr, size_t bytes, cudaStream_
 
 // One device allocation per scene, 256-byte aligned sub-buffers in this
 // order: BVH2 nodes, BVH4 nodes, records, triangles, planes, parent links of
-// BVH2 and BVH4, refit words, BVH8 nodes, BVH8 slot sources, grid nodes, the
-// grid.  Fills every
-// pointer and count of the scene from `info` and the node counts; the
-// contents are the caller's to write.
+// BVH2 and BVH4, refit words, BVH8 nodes, BVH8 slot sources, grid nodes (none
+// without grid_fits), the grid.  Fills every pointer and count of the scene
+// from `info` and the node counts; the contents are the caller's to write.
 igxrt_status allocate_scene(igxrt_context* ctx, const igxrt_bvh_info& info, uint32_t n2, uint32_t n4,
                             uint32_t n8, igxrt_scene*& out, bool pool, cudaStream_t stream) {
     out = nullptr;
@@ -121,7 +120,8 @@ igxrt_status allocate_scene(igxrt_context* ctx, const igxrt_bvh_info& info, uint
     const size_t b8 = round_up((size_t)n8 * sizeof(igxrt_bvh8_node), 256);
     const size_t bs8 = round_up((size_t)n8 * 8 * sizeof(uint32_t), 256);
     const size_t o8 = b2 + b4 + bp + bt + bl + bpar + bw;
-    const size_t og = o8 + b8 + bs8, bg = (size_t)n4 * 4 * sizeof(float4);
+    s->grid_fits = records <= ctx->grid_records;
+    const size_t og = o8 + b8 + bs8, bg = s->grid_fits ? (size_t)n4 * 4 * sizeof(float4) : 0;
     const size_t bytes = og + bg + 2 * sizeof(float4);
     bool pooled = false;
     cudaError_t e = pool ? pool_alloc(ctx, &s->d_mem, bytes, stream, pooled) : cudaMalloc(&s->d_mem, bytes);
@@ -133,7 +133,7 @@ igxrt_status allocate_scene(igxrt_context* ctx, const igxrt_bvh_info& info, uint
     }
     char* base = (char*)s->d_mem;
     s->grid_nodes = (float4*)(base + og);
-    s->grid = s->grid_nodes + 4 * (size_t)n4;
+    s->grid = (float4*)(base + og + bg);
     s->nodes[IGXRT_LAYOUT_BVH8] = base + o8;
     s->node_count[IGXRT_LAYOUT_BVH8] = n8;
     s->src8 = (const uint32_t*)(base + o8 + b8);

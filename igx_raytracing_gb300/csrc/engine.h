@@ -50,6 +50,9 @@ struct igxrt_context {
     // at the next synchronisation, the rest when the context and the last
     // scene are gone.  Null where the device has no pools.
     std::shared_ptr<igxrt::MemoryPool> pool;
+    // Largest scene, in records, that gets grid nodes (2^27, the leaf
+    // references' field; tests lower it: igxrt_internal_set_grid_records).
+    uint64_t grid_records = 1ull << 27;
     // The device loads and stores pageable host memory through the host's
     // page tables (cudaDevAttrPageableMemoryAccessUsesHostPageTables).
     bool pageable_access = false;
@@ -80,6 +83,9 @@ struct igxrt_scene {
     float4* grid_nodes = nullptr;
     float4* grid = nullptr;
     bool grid_ok = false;
+    // every record fits a grid leaf's reference: the scene's size, so a refit
+    // does not change it
+    bool grid_fits = false;
     // BVH8 slots' sources in the BVH2 layout (8 per BVH8 node), for the refit
     const uint32_t* src8 = nullptr;
     // GPU refit scratch, two float4 per record ({box lo, leaf_end}, {box hi,
@@ -126,6 +132,8 @@ igxrt_status allocate_scene(igxrt_context* ctx, const igxrt_bvh_info& info, uint
 // Queues the kernel that writes the scene's grid nodes and folds its findings
 // into the refit words kGridWord* (zeroed before); grid_usable judges the
 // words once they are on the host.
+// Scenes without grid_fits get none, at creation and at every refit alike:
+// the words stay zero, which grid_usable refuses.
 cudaError_t write_grid_nodes(const igxrt_context* ctx, const igxrt_scene* scene, bool refit, cudaStream_t stream);
 bool grid_usable(const uint32_t* words);
 // Launches over a scene with grid nodes use them in place of the two layouts
@@ -274,3 +282,12 @@ class DeviceGuard {
 };
 
 }  // namespace igxrt
+
+// Entry points for the tests, in no public header: which nodes the scene's
+// BVH2 and BVH4 launches trace now (1: grid nodes, 0: exact), and a context's
+// limit on the records of a scene with grid nodes, for scenes created after
+// the call (0: every scene stays on the exact nodes for its life).
+extern "C" {
+uint32_t igxrt_internal_uses_grid(const igxrt_scene* scene);
+void igxrt_internal_set_grid_records(igxrt_context* ctx, uint64_t records);
+}

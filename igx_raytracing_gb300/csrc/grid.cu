@@ -107,10 +107,8 @@ __global__ void __launch_bounds__(128) grid_nodes_kernel(const igxrt_bvh4_node* 
             } else {
                 const uint32_t first = ~(uint32_t)ref;
                 uint32_t more = 0;
-                while (!prims[first + more].leaf_end)
+                while (!prims[first + more].leaf_end)  // at most 16 records
                     ++more;
-                if (more > 15u || first >= (1u << 27))  // the reference's fields
-                    atomicOr(words + kGridWordUnfit, 1u);
                 child = kGridLeaf | (first << 4) | (more & 15u);
             }
             Box q;
@@ -148,7 +146,7 @@ __global__ void __launch_bounds__(128) grid_nodes_kernel(const igxrt_bvh4_node* 
 
 cudaError_t write_grid_nodes(const igxrt_context* ctx, const igxrt_scene* s, bool refit, cudaStream_t stream) {
     const uint32_t n4 = s->node_count[IGXRT_LAYOUT_BVH4];
-    if (!n4)
+    if (!n4 || !s->grid_fits)
         return cudaSuccess;
     const igxrt_bvh4_node* nodes = static_cast<const igxrt_bvh4_node*>(s->nodes[IGXRT_LAYOUT_BVH4]);
     // two rounds of blocks at most: each ends in two atomics on the same words
@@ -161,8 +159,8 @@ cudaError_t write_grid_nodes(const igxrt_context* ctx, const igxrt_scene* s, boo
     return cudaGetLastError();
 }
 
-// The rule that decides whether launches use the grid nodes: every leaf fits
-// a reference, and the slots' surface areas grew by the quantization to at
+// The rule that decides whether launches use the grid nodes: they were written
+// (write_grid_nodes), and the slots' surface areas grew by the quantization to at
 // most kGridGrowth times on average (a ray visits boxes about in proportion
 // to their area).  The mean over the slots, not over the area: a scene whose
 // detail is smaller than the grid's steps, however small a part of its area,
@@ -174,3 +172,11 @@ bool grid_usable(const uint32_t* words) {
 }
 
 }  // namespace igxrt
+
+extern "C" {
+
+uint32_t igxrt_internal_uses_grid(const igxrt_scene* scene) { return igxrt::use_grid(*scene, IGXRT_LAYOUT_BVH2); }
+
+void igxrt_internal_set_grid_records(igxrt_context* ctx, uint64_t records) { ctx->grid_records = records; }
+
+}  // extern "C"
