@@ -217,7 +217,7 @@ __global__ void __maxnreg__(batch_kernel_regs(LAYOUT, MIXED)) batch_kernel(Batch
                     occluded = mode ? process_leaf<true, false>(prims, next, r, best, unused)
                                     : process_leaf<false, false>(prims, next, r, best, unused);
                 if (!occluded)
-                    next = st.pop_live(best.tcull);
+                    next = GRID ? st.pop_split(best.tcull) : st.pop_live(best.tcull);
             }
             if (overflow)
                 atomicOr(a.status, kStatusStackOverflow);

@@ -118,7 +118,7 @@ __device__ __forceinline__ int32_t visit_grid(const float4* __restrict__ nodes, 
         c[k] = __float_as_int(s[k].w);
     }
     if (m == 0)
-        return st.pop_live(tcull);
+        return st.pop_split(tcull);
     grid_order(t[0], t[1], c[0], c[1]);
     grid_order(t[2], t[3], c[2], c[3]);
     grid_order(t[0], t[2], c[0], c[2]);

@@ -151,7 +151,7 @@ __device__ __forceinline__ void warp_leaf_phase(const float4* __restrict__ prims
     }
     __syncwarp();  // the list is free again
     if (at_leaf && !occluded)
-        next = st.pop_live(best.tcull);
+        next = st.pop_split(best.tcull);
 }
 
 }  // namespace igxrt

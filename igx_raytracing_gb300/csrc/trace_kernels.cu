@@ -277,7 +277,7 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
                            : MIXED ? process_leaf_mixed<ANY, COUNT>(a.prims, next, r, best, &pf)
                                    : process_leaf<ANY, COUNT>(a.prims, next, r, best, pf);
                 if (!occluded)
-                    next = st.pop_live(best.tcull);
+                    next = GRID ? st.pop_split(best.tcull) : st.pop_live(best.tcull);
             }
             if (overflow)
                 atomicOr(a.status, kStatusStackOverflow);
