@@ -208,8 +208,7 @@ __global__ void __maxnreg__(batch_kernel_regs(LAYOUT, MIXED)) batch_kernel(Batch
             occluded_at_start = false;
             if (next < 0) {
                 if (GRID)
-                    occluded = mode ? process_grid_leaf<true, MIXED>(prims, next, r, best)
-                                    : process_grid_leaf<false, MIXED>(prims, next, r, best);
+                    occluded = process_grid_leaf<MIXED>(prims, next, r, best, mode != 0u);
                 else if (MIXED)
                     occluded = mode ? process_leaf_mixed<true>(prims, next, r, best)
                                     : process_leaf_mixed<false>(prims, next, r, best);

@@ -45,8 +45,25 @@ __device__ __forceinline__ uint32_t grid_near(float step) {
     return kPickLo ^ ((uint32_t)(__float_as_int(step) >> 31) & kPickSwap);
 }
 
+// What an axis' plane distances are widened by at either end, in units of the
+// origin's distance along it.  The folded origin is rounded to 2^-24 of that
+// distance three times (1/dir, its product with the origin, the sum with the
+// grid's), and the triangle test's own rounding moves a hit point by as much.
+// The boxes' padding covers that up to some 60 scene sizes; from farther out
+// rays at edges missed boxes of triangles that they hit: of 200,000 such hits
+// 15 at 200 scene sizes and 700 at 1,000 (over the exact nodes, which have the
+// same limit, 180 and 1,550), and none with this.  Within 10 scene sizes it is
+// less than half a word's step, and the multiply-adds cost at most 0.4%.
+constexpr float kGridSlack = 0x1p-22f;
+
+// The intercept of the far planes, from that of the near ones (to_grid), made
+// anew at every visit: kept in registers of the ray, the three cost the closest-hit
+// kernels more (the 1M sphere's step 905 us, 868 so).
+__device__ __forceinline__ float grid_far(float oi) { return __fmaf_rn(fabsf(oi), -2.f * kGridSlack, oi); }
+
 // Folds the scene's grid ({scale}, {origin}) into the ray's slab terms: the
-// distance to a plane word of axis a is then fmaf(value, ia, -oia).  An axis
+// distance to a plane word of axis a is then fmaf(value, ia, -oia), with oia
+// widened for the near planes and grid_far(oia) for the far ones.  An axis
 // whose step leaves the range in which that arithmetic is as precise as the
 // exact layouts' (a direction beyond 2^90 or so, or an axis-parallel ray in a
 // scene beyond 2^40) is taken out of the test: its distances are NaN, which
@@ -57,6 +74,7 @@ __device__ __forceinline__ void to_grid(RayState& r, const float4* __restrict__ 
     const auto axis = [](float& i, float& oi, float scale, float origin) {
         const float step = __fmul_rn(scale, i);
         oi = __fmaf_rn(-origin, i, oi);
+        oi = __fmaf_rn(fabsf(oi), kGridSlack, oi);
         i = fabsf(step) >= 0x1p-108f && fabsf(step) <= 0x1p108f ? step : __int_as_float(0x7fffffff);
     };
     axis(r.ix, r.oix, s.x, o.x);
@@ -66,14 +84,14 @@ __device__ __forceinline__ void to_grid(RayState& r, const float4* __restrict__ 
 }
 
 template <bool MIXED>
-__device__ __forceinline__ bool grid_box_test(const RayState& r, uint32_t sx, uint32_t sy, uint32_t sz, float x,
+__device__ __forceinline__ bool grid_box_test(const RayState& r, float ofx, float ofy, float ofz, uint32_t sx, uint32_t sy, uint32_t sz, float x,
                                               float y, float z, float tcull, float& tn) {
     const float nx = __fmaf_rn(grid_plane(x, sx), r.ix, -r.oix);
-    const float fx = __fmaf_rn(grid_plane(x, sx ^ kPickSwap), r.ix, -r.oix);
+    const float fx = __fmaf_rn(grid_plane(x, sx ^ kPickSwap), r.ix, -ofx);
     const float ny = __fmaf_rn(grid_plane(y, sy), r.iy, -r.oiy);
-    const float fy = __fmaf_rn(grid_plane(y, sy ^ kPickSwap), r.iy, -r.oiy);
+    const float fy = __fmaf_rn(grid_plane(y, sy ^ kPickSwap), r.iy, -ofy);
     const float nz = __fmaf_rn(grid_plane(z, sz), r.iz, -r.oiz);
-    const float fz = __fmaf_rn(grid_plane(z, sz ^ kPickSwap), r.iz, -r.oiz);
+    const float fz = __fmaf_rn(grid_plane(z, sz ^ kPickSwap), r.iz, -ofz);
     if (MIXED) {
         // the bounds by FLT_MAX count only when all three axes are out of the test
         const float tnear = fmaxf(fmaxf(nx, ny), fmaxf(nz, -3.4028235e38f));
@@ -107,18 +125,19 @@ __device__ __forceinline__ int32_t visit_grid(const float4* __restrict__ nodes, 
     ldg256(n, s[0], s[1]);
     ldg256(n + 2, s[2], s[3]);
     const uint32_t sx = grid_near(r.ix), sy = grid_near(r.iy), sz = grid_near(r.iz);
+    const float ofx = grid_far(r.oix), ofy = grid_far(r.oiy), ofz = grid_far(r.oiz);
     int32_t t[4], c[4];
     uint32_t m = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         float tn;
-        const bool hit = grid_box_test<MIXED>(r, sx, sy, sz, s[k].x, s[k].y, s[k].z, tcull, tn);
+        const bool hit = grid_box_test<MIXED>(r, ofx, ofy, ofz, sx, sy, sz, s[k].x, s[k].y, s[k].z, tcull, tn);
         m += hit ? 1u : 0u;
         t[k] = hit ? __float_as_int(tn) : kMiss;
         c[k] = __float_as_int(s[k].w);
     }
     if (m == 0)
-        return st.pop_split(tcull);
+        return st.pop_live(tcull);
     grid_order(t[0], t[1], c[0], c[1]);
     grid_order(t[2], t[3], c[2], c[3]);
     grid_order(t[0], t[2], c[0], c[2]);
@@ -156,14 +175,16 @@ __device__ __forceinline__ int32_t visit_grid(const float4* __restrict__ nodes, 
 }
 
 // The leaf `ref` of a grid node.  Returns true when an any-hit query is decided.
-template <bool ANY, bool MIXED>
+// `any` may differ between lanes (the batch kernel): one loop for both kinds of
+// query, since a loop for each made the batch kernel 8% slower (328 us, 304 so).
+template <bool MIXED>
 __device__ __forceinline__ bool process_grid_leaf(const float4* __restrict__ prims, int32_t ref, const RayState& r,
-                                                  BestHit& best) {
+                                                  BestHit& best, bool any) {
     uint32_t i = ((uint32_t)ref & ~kGridLeaf) >> 4;
     const float4* p = prims + 3 * (size_t)i;
     for (int32_t more = ref & 15;; --more, ++i, p += 3) {
         const float4 v0 = __ldg(p), v1 = __ldg(p + 1), v2 = __ldg(p + 2);
-        if ((MIXED ? test_record_mixed<ANY>(v0, v1, v2, i, r, best) : test_record<ANY>(v0, v1, v2, r, best)) && ANY)
+        if ((MIXED ? test_record_mixed(v0, v1, v2, i, r, best, any) : test_record(v0, v1, v2, r, best, any)) && any)
             return true;
         if (more == 0)
             return false;

@@ -114,7 +114,7 @@ __device__ __forceinline__ void warp_leaf_phase(const float4* __restrict__ prims
             q.prev = skip;
             if (ANY) {
                 BestHit unused;
-                found = test_record<true>(v0, v1, v2, q, unused);
+                found = test_record(v0, v1, v2, q, unused, true);
             } else {
                 float t, u, v;
                 if (tri_test(q, v0, v1, v2, t, u, v) && t <= limit && !(t <= q.tmin)) {

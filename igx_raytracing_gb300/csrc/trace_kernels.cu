@@ -108,9 +108,10 @@ __device__ __forceinline__ void flush_uv(const KernelArgs& a, uint32_t* batch, u
 // without spills than with more warps: 56, 60, 64 and 72 registers take 2,553,
 // 2,586, 2,398 and 2,442 us on 4M incoherent rays over 2M triangles, and 461,
 // 452, 440 and 438 us on the 1M sphere's 1080p primaries.  The any-hit kernel
-// gains from 72 (1M occlusion rays 356 us, 364 at 64).
+// gains from 72 (1M occlusion rays 356 us, 364 at 64), and so does the
+// closest-hit kernel of mixed scenes (1M rays 591 us, 628 at 64).
 constexpr int trace_kernel_regs(int layout, bool any, bool mixed) {
-    return layout == (int)kLayoutGrid    ? (any && !mixed ? 72 : 64)
+    return layout == (int)kLayoutGrid    ? (any != mixed ? 72 : 64)
            : layout == IGXRT_LAYOUT_BVH2 ? (mixed && !any ? 64 : 56)
            : layout == IGXRT_LAYOUT_BVH4 ? (mixed && !any ? 72 : 64)
                                          : (any && !mixed ? 64 : 80);
@@ -273,7 +274,7 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
             occluded_at_start = false;
             // leaf phase
             if (!WARP_LEAVES && next < 0) {
-                occluded = GRID    ? process_grid_leaf<ANY, MIXED>(a.prims, next, r, best)
+                occluded = GRID    ? process_grid_leaf<MIXED>(a.prims, next, r, best, ANY)
                            : MIXED ? process_leaf_mixed<ANY, COUNT>(a.prims, next, r, best, &pf)
                                    : process_leaf<ANY, COUNT>(a.prims, next, r, best, pf);
                 if (!occluded)

@@ -212,17 +212,16 @@ struct TraversalStack {
 constexpr uint32_t kStackEntryBytes = 8;
 
 // One triangle record against the ray.  Returns true when an any-hit query is
-// decided (ANY), or when the record became the best hit (closest).
-template <bool ANY>
+// decided (`any`), or when the record became the best hit (closest).
 __device__ __forceinline__ bool test_record(const float4& v0, const float4& v1, const float4& v2,
-                                            const RayState& r, BestHit& best) {
+                                            const RayState& r, BestHit& best, bool any) {
     float t, u, v;
     if (!tri_test(r, v0, v1, v2, t, u, v))
         return false;
     const uint32_t prim = __float_as_uint(v0.w);
     if (t <= r.tmin || prim == r.prev)
         return false;
-    if (ANY)
+    if (any)
         return t < r.tmax_eff;
     if (!(t < best.t || (t == best.t && prim < best.prim)))
         return false;
@@ -245,7 +244,7 @@ __device__ __forceinline__ bool process_leaf(const float4* __restrict__ prims, i
         const float4 v0 = __ldg(p), v1 = __ldg(p + 1), v2 = __ldg(p + 2);
         if (COUNT)
             ++pf;
-        if (test_record<ANY>(v0, v1, v2, r, best) && ANY)
+        if (test_record(v0, v1, v2, r, best, ANY) && ANY)
             return true;
         if (__float_as_uint(v1.w))
             break;
@@ -674,12 +673,11 @@ __device__ __forceinline__ void finish_uv(const float4* __restrict__ prims, cons
 }
 
 // Record `i` of a mixed scene against the ray.  Returns true when an any-hit
-// query is decided (ANY), or when the record became the best hit (closest).
+// query is decided (`any`), or when the record became the best hit (closest).
 // best_rec (optional): the record index of the best hit so far, for callers
 // that need the hit object's record afterwards (the G-buffer's normals).
-template <bool ANY>
 __device__ __forceinline__ bool test_record_mixed(const float4& v0, const float4& v1, const float4& v2,
-                                                  uint32_t i, const RayState& r, BestHit& best,
+                                                  uint32_t i, const RayState& r, BestHit& best, bool any,
                                                   uint32_t* best_rec = nullptr) {
     const uint32_t type = __float_as_uint(v2.w), id = __float_as_uint(v0.w);
     if (id == r.prev)
@@ -688,7 +686,7 @@ __device__ __forceinline__ bool test_record_mixed(const float4& v0, const float4
         float t, u, v;
         if (!tri_test(r, v0, v1, v2, t, u, v) || t <= r.tmin)
             return false;
-        if (ANY)
+        if (any)
             return t < r.tmax_eff;
         if (!better(t, prio_other(id), best))
             return false;
@@ -700,7 +698,7 @@ __device__ __forceinline__ bool test_record_mixed(const float4& v0, const float4
         float t;
         if (!sphere_hit(r, v0.x, v0.y, v0.z, v1.x, t) || !(t >= r.tmin))
             return false;
-        if (ANY)
+        if (any)
             return t < r.tmax_eff;
         if (!better(t, prio_other(id), best))
             return false;
@@ -713,7 +711,7 @@ __device__ __forceinline__ bool test_record_mixed(const float4& v0, const float4
         int axis;
         if (!cube_hit(r, v0, v1, t, axis))
             return false;
-        if (ANY)
+        if (any)
             return t < r.tmax_eff;
         if (!better(t, prio_cube(id), best))
             return false;
@@ -739,7 +737,7 @@ __device__ __forceinline__ bool process_leaf_mixed(const float4* __restrict__ pr
         const float4 v0 = __ldg(p), v1 = __ldg(p + 1), v2 = __ldg(p + 2);
         if (COUNT)
             ++*pf;
-        if (test_record_mixed<ANY>(v0, v1, v2, i, r, best, best_rec) && ANY)
+        if (test_record_mixed(v0, v1, v2, i, r, best, ANY, best_rec) && ANY)
             return true;
         if (__float_as_uint(v1.w))
             break;
