@@ -269,16 +269,20 @@ void batch_item_for(const igxrt_scene* scene, uint32_t layout, const igxrt_ray* 
     d.plane_base = scene->plane_base;
 }
 
+uint32_t batch_layout(const igxrt_batch_item* items, uint32_t count, uint32_t layout) {
+    for (uint32_t i = 0; i < count; ++i)
+        if (items[i].scene && !grid_or_empty(*items[i].scene, layout))
+            return layout;
+    return kLayoutGrid;
+}
+
 igxrt_status build_batch_table(igxrt_context* ctx, const igxrt_batch_item* items, uint32_t count,
                                const igxrt_launch_params& p, std::vector<BatchItemDev>& table,
                                uint32_t& total_packets, uint64_t& total_rays, bool& mixed,
                                uint32_t& layout) {
     if (count && !items)
         return fail(ctx, IGXRT_ERROR_INVALID_ARGUMENT, "items is NULL");
-    layout = kLayoutGrid;
-    for (uint32_t i = 0; i < count; ++i)
-        if (items[i].scene && !use_grid(*items[i].scene, p.layout))
-            layout = p.layout;
+    layout = batch_layout(items, count, p.layout);
     table.resize(count);
     uint64_t packets = 0;
     total_rays = 0;
@@ -391,13 +395,96 @@ igxrt_status batch_slot(igxrt_context* ctx, uint32_t count, BatchItemDev** slot,
 
 using namespace igxrt;
 
-struct igxrt_batch {
-    igxrt_context* ctx = nullptr;
+// A batch's captured launch over one kind of nodes.
+struct BatchForm {
+    bool ready = false;
     void* d_mem = nullptr;  // item table + queue word
     cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    uint64_t total_rays = 0;
+    cudaGraphExec_t exec = nullptr;  // null: no rays
 };
+
+struct igxrt_batch {
+    igxrt_context* ctx = nullptr;
+    igxrt_launch_params params{};
+    std::vector<igxrt_batch_item> items;
+    std::vector<const igxrt_scene*> scenes;  // the items', each once
+    // Over the named layout, and over the grid nodes.  A refit may take a
+    // scene's grid nodes out of use or bring them back (grid_usable), and each
+    // launch follows: the other form is captured when it is first wanted.
+    BatchForm forms[2];
+    uint32_t last = 0;  // the form of the latest launch
+};
+
+namespace {
+
+void release(BatchForm& f) {
+    if (f.exec)
+        cudaGraphExecDestroy(f.exec);
+    if (f.graph)
+        cudaGraphDestroy(f.graph);
+    if (f.d_mem)
+        cudaFree(f.d_mem);
+    f = BatchForm();
+}
+
+// The form that the batch's scenes allow now.
+uint32_t wanted_form(const igxrt_batch& b) {
+    for (const igxrt_scene* s : b.scenes)
+        if (!grid_or_empty(*s, b.params.layout))
+            return 0u;
+    return 1u;
+}
+
+// Uploads the item table and captures the launch of the form that the scenes
+// allow now, into b->forms[wanted_form].
+igxrt_status capture_form(igxrt_batch* b) {
+    igxrt_context* ctx = b->ctx;
+    const uint32_t count = (uint32_t)b->items.size();
+    std::vector<BatchItemDev> table;
+    uint32_t packets = 0;
+    uint64_t rays = 0;
+    bool mixed = false;
+    uint32_t layout = b->params.layout;
+    igxrt_status st = build_batch_table(ctx, b->items.data(), count, b->params, table, packets, rays, mixed, layout);
+    if (st != IGXRT_OK)
+        return st;
+    BatchForm& f = b->forms[layout == kLayoutGrid ? 1 : 0];
+    const size_t tb = (table.size() * sizeof(BatchItemDev) + 255) / 256 * 256;
+    cudaError_t e = cudaMalloc(&f.d_mem, tb + 256);
+    if (e == cudaSuccess && !table.empty())
+        e = cudaMemcpy(f.d_mem, table.data(), table.size() * sizeof(BatchItemDev), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+        release(f);
+        return cuda_fail(ctx, e, "batch table");
+    }
+    uint32_t* queue = reinterpret_cast<uint32_t*>(static_cast<char*>(f.d_mem) + tb);
+    cudaStream_t cap = nullptr;
+    e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
+    if (e == cudaSuccess)
+        e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+        st = launch_batch(ctx, static_cast<const BatchItemDev*>(f.d_mem), count, packets, rays, b->params,
+                          queue, cap, mixed, layout);
+        const cudaError_t e2 = cudaStreamEndCapture(cap, &f.graph);
+        if (st == IGXRT_OK && e2 != cudaSuccess)
+            st = cuda_fail(ctx, e2, "batch graph capture");
+        if (st == IGXRT_OK && f.graph) {
+            e = cudaGraphInstantiate(&f.exec, f.graph, 0);
+            if (e != cudaSuccess)
+                st = cuda_fail(ctx, e, "batch graph instantiate");
+        }
+    } else {
+        st = cuda_fail(ctx, e, "batch capture stream");
+    }
+    if (cap)
+        cudaStreamDestroy(cap);
+    if (st != IGXRT_OK)
+        release(f);
+    f.ready = st == IGXRT_OK;
+    return st;
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -453,55 +540,26 @@ igxrt_status igxrt_batch_create(igxrt_context* ctx, const igxrt_batch_item* item
     igxrt_status st = resolve_params(ctx, params ? *params : ctx->params, p);
     if (st != IGXRT_OK)
         return st;
-    std::vector<BatchItemDev> table;
-    uint32_t packets = 0;
-    uint64_t rays = 0;
-    bool mixed = false;
-    uint32_t layout = p.layout;
-    st = build_batch_table(ctx, items, count, p, table, packets, rays, mixed, layout);
-    if (st != IGXRT_OK)
-        return st;
+    if (count && !items)
+        return fail(ctx, IGXRT_ERROR_INVALID_ARGUMENT, "items is NULL");
     DeviceGuard guard(ctx->device);
     if (!guard.ok())
         return fail(ctx, IGXRT_ERROR_CUDA, "cannot select the context's device");
     igxrt_batch* b = new (std::nothrow) igxrt_batch();
     if (!b)
         return fail(ctx, IGXRT_ERROR_OUT_OF_MEMORY, "batch object");
-    b->ctx = ctx;
-    b->total_rays = rays;
-    const size_t tb = (table.size() * sizeof(BatchItemDev) + 255) / 256 * 256;
-    cudaError_t e = cudaMalloc(&b->d_mem, tb + 256);
-    if (e == cudaSuccess && !table.empty())
-        e = cudaMemcpy(b->d_mem, table.data(), table.size() * sizeof(BatchItemDev), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-        if (b->d_mem)
-            cudaFree(b->d_mem);
-        delete b;
-        return cuda_fail(ctx, e, "batch table");
+    try {
+        b->ctx = ctx;
+        b->params = p;
+        b->items.assign(items, items + count);
+        st = capture_form(b);  // refuses items without a scene
+        for (uint32_t i = 0; i < count && st == IGXRT_OK; ++i)
+            b->scenes.push_back(items[i].scene);
+        std::sort(b->scenes.begin(), b->scenes.end());
+        b->scenes.erase(std::unique(b->scenes.begin(), b->scenes.end()), b->scenes.end());
+    } catch (const std::bad_alloc&) {
+        st = fail(ctx, IGXRT_ERROR_OUT_OF_MEMORY, "batch table");
     }
-    uint32_t* queue = reinterpret_cast<uint32_t*>(static_cast<char*>(b->d_mem) + tb);
-    cudaStream_t cap = nullptr;
-    e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
-    if (e == cudaSuccess)
-        e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        st = launch_batch(ctx, static_cast<const BatchItemDev*>(b->d_mem), count, packets, rays, p,
-                          queue, cap, mixed, layout);
-        cudaGraph_t g = nullptr;
-        const cudaError_t e2 = cudaStreamEndCapture(cap, &g);
-        b->graph = g;
-        if (st == IGXRT_OK && e2 != cudaSuccess)
-            st = cuda_fail(ctx, e2, "batch graph capture");
-        if (st == IGXRT_OK && b->graph) {
-            e = cudaGraphInstantiate(&b->exec, b->graph, 0);
-            if (e != cudaSuccess)
-                st = cuda_fail(ctx, e, "batch graph instantiate");
-        }
-    } else {
-        st = cuda_fail(ctx, e, "batch capture stream");
-    }
-    if (cap)
-        cudaStreamDestroy(cap);
     if (st != IGXRT_OK) {
         igxrt_batch_destroy(b);
         return st;
@@ -513,10 +571,22 @@ igxrt_status igxrt_batch_create(igxrt_context* ctx, const igxrt_batch_item* item
 igxrt_status igxrt_batch_launch(igxrt_batch* b, void* stream) {
     if (!b)
         return IGXRT_ERROR_INVALID_ARGUMENT;
-    if (!b->exec)
-        return IGXRT_OK;  // an empty batch captured nothing
     DeviceGuard guard(b->ctx->device);
-    const cudaError_t e = cudaGraphLaunch(b->exec, (cudaStream_t)stream);
+    uint32_t form = wanted_form(*b);
+    if (!b->forms[form].ready) {
+        // both forms find the same hits: without the memory for the other, the
+        // one there is serves
+        try {
+            if (capture_form(b) != IGXRT_OK)
+                form ^= 1u;
+        } catch (const std::bad_alloc&) {
+            form ^= 1u;
+        }
+    }
+    b->last = form;
+    if (!b->forms[form].exec)
+        return IGXRT_OK;  // an empty batch captured nothing
+    const cudaError_t e = cudaGraphLaunch(b->forms[form].exec, (cudaStream_t)stream);
     if (e != cudaSuccess)
         return cuda_fail(b->ctx, e, "batch graph launch");
     return IGXRT_OK;
@@ -528,15 +598,13 @@ igxrt_status igxrt_batch_destroy(igxrt_batch* b) {
     {
         DeviceGuard guard(b->ctx->device);
         cudaDeviceSynchronize();
-        if (b->exec)
-            cudaGraphExecDestroy(b->exec);
-        if (b->graph)
-            cudaGraphDestroy(b->graph);
-        if (b->d_mem)
-            cudaFree(b->d_mem);
+        release(b->forms[0]);
+        release(b->forms[1]);
     }
     delete b;
     return IGXRT_OK;
 }
+
+uint32_t igxrt_internal_batch_uses_grid(const igxrt_batch* batch) { return batch->last; }
 
 }  // extern "C"

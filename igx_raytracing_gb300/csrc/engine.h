@@ -142,6 +142,10 @@ bool grid_usable(const uint32_t* words);
 // sphere's primaries 471 -> 440 us, 4M incoherent rays over 2M triangles
 // 3,003 -> 2,398 us).  BVH8 stays as named.
 inline bool use_grid(const igxrt_scene& s, uint32_t layout) { return s.grid_ok && layout != IGXRT_LAYOUT_BVH8; }
+// A scene without nodes takes part in any launch.
+inline bool grid_or_empty(const igxrt_scene& s, uint32_t layout) {
+    return use_grid(s, layout) || (layout != IGXRT_LAYOUT_BVH8 && s.node_count[layout] == 0);
+}
 
 // Parent links of both layouts, computed on the host at scene creation and
 // stored after the scene's other buffers (see refit.cu).
@@ -212,11 +216,13 @@ struct BatchItemDev {
     uint32_t plane_base;    // object id of the scene's first plane
 };
 
+// Node layout of one launch over all items: kLayoutGrid when every item's
+// scene allows it (grid_or_empty), else the named one.
+uint32_t batch_layout(const igxrt_batch_item* items, uint32_t count, uint32_t layout);
 // Fills the device table of `count` items; `mixed` is set when an item's
 // scene holds spheres, cubes or planes (the batch then runs the mixed kernel,
 // which traces triangle-only items as well), `layout` to the nodes the table
-// points at: kLayoutGrid when every item's scene has them (use_grid), else
-// p.layout.
+// points at (batch_layout).
 igxrt_status build_batch_table(igxrt_context* ctx, const igxrt_batch_item* items, uint32_t count,
                                const igxrt_launch_params& p, std::vector<BatchItemDev>& table,
                                uint32_t& total_packets, uint64_t& total_rays, bool& mixed,
@@ -290,4 +296,6 @@ class DeviceGuard {
 extern "C" {
 uint32_t igxrt_internal_uses_grid(const igxrt_scene* scene);
 void igxrt_internal_set_grid_records(igxrt_context* ctx, uint64_t records);
+// The nodes of a batch's latest launch (1: grid nodes).
+uint32_t igxrt_internal_batch_uses_grid(const igxrt_batch* batch);
 }

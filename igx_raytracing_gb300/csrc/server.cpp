@@ -201,7 +201,7 @@ bool igxrt_server::launch_one() {
         igxrt_ray* d_rays = reinterpret_cast<igxrt_ray*>(base) + first;
         uint32_t* d_prev = q->r.prev_hit ? reinterpret_cast<uint32_t*>(base + rb) + first : nullptr;
         BatchItemDev& d = s->h_table[s->slices.size()];
-        if (!use_grid(*sc, params.layout) && layout == kLayoutGrid) {
+        if (!grid_or_empty(*sc, params.layout) && layout == kLayoutGrid) {
             layout = params.layout;
             for (size_t k = 0; k < s->slices.size(); ++k) {
                 const igxrt_scene* other = scenes[s->slices[k].q->r.scene_id];

@@ -457,7 +457,10 @@ typedef struct igxrt_batch igxrt_batch;
  * item table is uploaded once and the queue reset plus the kernel are
  * captured in a CUDA graph; igxrt_batch_launch replays it.  params NULL
  * takes the context's launch parameters.  Results are identical to tracing
- * each item on its own.
+ * each item on its own.  The scenes and arrays must outlive the batch's last
+ * launch.  A refit may move a scene between the layout's nodes and their
+ * quantized form (igxrt_launch_params.layout); the next launch of the batch
+ * follows and captures its graph anew the first time that happens.
  */
 igxrt_status igxrt_batch_create(igxrt_context* ctx, const igxrt_batch_item* items, uint32_t count,
                                 const igxrt_launch_params* params, igxrt_batch** out);

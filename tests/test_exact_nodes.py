@@ -9,6 +9,7 @@ import pytest
 
 import igx_raytracing_gb300 as igx
 from igx_raytracing_gb300 import scenes
+from igx_raytracing_gb300._capi import HIT_DTYPE
 from oracle import pyoracle
 
 pytestmark = pytest.mark.gpu
@@ -60,3 +61,45 @@ def test_a_refit_keeps_a_scene_too_large_for_the_references(gpu_build):
             _check(scene, t, rays, f"{n} records")
         scene.close()
     ctx.close()
+
+
+def _far(tris):
+    """One vertex far away: the grid's steps outgrow the other triangles."""
+    out = tris.copy()
+    out["p0"][7] += np.float32(3e6)
+    return out
+
+
+@pytest.mark.parametrize("starts_fit", [True, False])
+def test_a_captured_batch_follows_its_scenes(ctx, starts_fit):
+    """A batch's launch traces the grid nodes exactly while every scene's can
+    serve, whichever way it was captured; an empty scene does not matter."""
+    import torch
+
+    a = scenes.random_triangles(3000, 8110, mu=math.log(0.03))
+    b = scenes.random_triangles(500, 8111, mu=math.log(0.05))
+    near, far = a, _far(a)
+    scene, other, empty = ctx.create_scene(near if starts_fit else far), ctx.create_scene(b), ctx.create_scene(a[:0])
+    rays = scenes.incoherent_rays(2000, 8112)
+    d_rays = _device(rays)
+    outs = [torch.empty(len(rays), 4, device="cuda") for _ in range(3)]
+    batch = ctx.create_batch([(s, d_rays, None, o, 0) for s, o in zip((scene, other, empty), outs)])
+    on_grid = lambda: bool(igx.lib().igxrt_internal_batch_uses_grid(batch._h))
+    for step, t in enumerate([None, far, near, near, far, near]):
+        if t is not None:
+            scene.refit(_device(t))
+        t = t if t is not None else (near if starts_fit else far)
+        assert uses_grid(scene) == (t is near), step
+        for o in outs:
+            o.fill_(-1)
+        batch.launch()
+        assert on_grid() == (t is near), step
+        torch.cuda.synchronize()
+        for tri, o in zip((t, b, a[:0]), outs):
+            got = o.cpu().numpy().view(HIT_DTYPE).reshape(-1)
+            expect, flags = pyoracle.trace_geometry(tri, rays)
+            for f in ("prim", "t", "u", "v"):
+                assert np.array_equal(got[f][flags == 0].view(np.uint32), expect[f][flags == 0].view(np.uint32)), (step, f)
+    batch.close()
+    for s in (scene, other, empty):
+        s.close()
