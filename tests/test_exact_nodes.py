@@ -103,3 +103,41 @@ def test_a_captured_batch_follows_its_scenes(ctx, starts_fit):
     batch.close()
     for s in (scene, other, empty):
         s.close()
+
+
+def _overflowing(tris):
+    """Two triangles whose distance along x is no float: the grid has no step
+    there."""
+    out = tris.copy()
+    for k, x in ((3, -2.5e38), (4, 2.5e38)):
+        out["p0"][k], out["p1"][k], out["p2"][k] = (x, 0, 0), (x, 1, 0), (x, 0, 1)
+    return out
+
+
+def test_a_captured_trace_over_a_range_that_overflows(ctx):
+    """A trace captured over grid nodes keeps them: a refit whose range is no
+    float takes that axis out of its box tests instead of losing hits."""
+    import torch
+
+    tris = scenes.random_triangles(500, 8115, mu=math.log(0.1))
+    rays = scenes.incoherent_rays(2000, 8116)
+    scene = ctx.create_scene(tris)
+    d_rays, out = _device(rays), torch.empty(len(rays), 4, device="cuda")
+    ctx.trace_closest(scene, d_rays, out=out)  # nothing is allocated in the capture
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ctx.trace_closest(scene, d_rays, out=out)
+    for t, grid in ((tris, True), (_overflowing(tris), False), (tris, True)):
+        scene.refit(_device(t))
+        assert uses_grid(scene) == grid
+        out.fill_(-1)
+        graph.replay()
+        torch.cuda.synchronize()
+        got = out.cpu().numpy().view(HIT_DTYPE).reshape(-1)
+        expect, flags = pyoracle.trace_geometry(t, rays)
+        ok = flags == 0
+        assert ok.mean() > 0.9 and (expect["prim"][ok] != 0xFFFFFFFF).mean() > 0.5
+        for f in ("prim", "t", "u", "v"):
+            assert np.array_equal(got[f][ok].view(np.uint32), expect[f][ok].view(np.uint32)), f
+    scene.close()
