@@ -24,7 +24,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = ["bvh_build.cpp", "capi.cpp", "autotune.cpp", "server.cpp", "trace_kernels.cu",
            "batch.cu", "shadow.cu", "gbuffer.cu", "grid.cu", "refit.cu", "lbvh.cu", "static_scratch.cu"]
 HEADERS = ["internal.h", "engine.h", "traverse.cuh", "geometry.cuh", "share.cuh", "gbuffer.cuh", "grid.cuh",
-           "leaf.cuh"]
+           "grid_write.cuh", "leaf.cuh"]
 
 
 def nvcc_path() -> str:

@@ -511,7 +511,7 @@ igxrt_status igxrt_scene_create_from_bvh(igxrt_context* ctx, const igxrt_bvh* bv
     if (e == cudaSuccess)
         e = cudaMemset(s->refit_words, 0, sizeof(words));
     if (e == cudaSuccess)
-        e = write_grid_nodes(ctx, s, false, nullptr);
+        e = write_grid_nodes(ctx, s, nullptr);
     if (e == cudaSuccess)
         e = cudaMemcpy(words, s->refit_words, sizeof(words), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess)

@@ -129,12 +129,12 @@ cudaError_t pool_alloc(igxrt_context* ctx, void** ptr, size_t bytes, cudaStream_
 igxrt_status allocate_scene(igxrt_context* ctx, const igxrt_bvh_info& info, uint32_t n2, uint32_t n4,
                             uint32_t n8, igxrt_scene*& out, bool pool = false, cudaStream_t stream = nullptr);
 
-// Queues the kernel that writes the scene's grid nodes and folds its findings
-// into the refit words kGridWord* (zeroed before); grid_usable judges the
-// words once they are on the host.
+// Queues the kernel that writes a new scene's grid nodes and folds its findings
+// into the refit words kGridWord* (zeroed before); a refit writes them itself
+// (refit.cu).  grid_usable judges the words once they are on the host.
 // Scenes without grid_fits get none, at creation and at every refit alike:
 // the words stay zero, which grid_usable refuses.
-cudaError_t write_grid_nodes(const igxrt_context* ctx, const igxrt_scene* scene, bool refit, cudaStream_t stream);
+cudaError_t write_grid_nodes(const igxrt_context* ctx, const igxrt_scene* scene, cudaStream_t stream);
 bool grid_usable(const uint32_t* words);
 // Launches over a scene with grid nodes use them in place of the two layouts
 // of exact boxes, whichever of the two the caller names: both find the same

@@ -710,7 +710,7 @@ igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* 
     if (e == cudaSuccess)
         e = cudaMemsetAsync(scene->refit_words, 0, kRefitStateWords * sizeof(uint32_t), s);
     if (e == cudaSuccess)
-        e = write_grid_nodes(ctx, scene, false, s);
+        e = write_grid_nodes(ctx, scene, s);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(w, scene->refit_words, kRefitStateWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)

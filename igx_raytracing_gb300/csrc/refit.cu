@@ -2,7 +2,7 @@
 //
 // The reference re-uploads its moving spheres every frame and traces them with
 // a linear loop (test/scene/niels_scene.cpp:61-70, res/shaders/trace.glsl:22-46);
-// over a BVH, moved geometry needs the node boxes to follow.  Five passes on
+// over a BVH, moved geometry needs the node boxes to follow.  Four passes on
 // the caller's stream:
 //   1. scan: bounds of every object, max |coordinate| (which sets the padding)
 //      and the scene box, reduced per block, then one atomicMax per block and
@@ -19,9 +19,9 @@
 //      atomic counter per node) writes the union of the slots into the
 //      parent's slot and climbs on; the others exit.  Nothing waits on another
 //      thread: a thread either continues or exits;
-//   4. BVH8: every compressed node re-quantized from the BVH2 boxes its slots
-//      were built from (eight lanes per node);
-//   5. grid nodes: the boxes re-quantized from the BVH4 nodes (grid.cu).
+//   4. quantized: every BVH8 node from the BVH2 boxes its slots were built from
+//      (eight lanes per node), every grid node from its BVH4 node
+//      (grid_write.cuh).
 // Boxes follow the host builder exactly (same min/max argument order, padded by
 // max(2^-18 * max|coordinate|, 1e-30)), so the GPU refit equals igxrt_bvh_refit
 // bit for bit.
@@ -30,6 +30,7 @@
 #include <algorithm>
 
 #include "geometry.cuh"
+#include "grid_write.cuh"
 
 namespace igxrt {
 
@@ -128,6 +129,9 @@ struct RefitArgs {
     const uint32_t* src8;
     uint32_t n8;
     float4* boxes;   // per record, in leaf order: {lo, leaf_end}, {hi, 0}
+    float4* grid_nodes;
+    float4* grid;
+    uint32_t grid_blocks;  // 0: the scene has no grid nodes
 };
 
 static_assert(kRefitStateWords >= 8, "the scan's words");
@@ -307,7 +311,7 @@ __global__ void refit_nodes_kernel(RefitArgs a) {
         refit_climb<IGXRT_LAYOUT_BVH4>(a, i - a.n2, pad);
 }
 
-// Pass 4: every BVH8 node re-quantized from the refit BVH2 boxes of its
+// Pass 4, BVH8: every node re-quantized from the refit BVH2 boxes of its
 // slots, eight lanes per node, one per slot.  The node's bounds are reduced
 // across the eight lanes with the lower slot as the first operand of every
 // comparison, which picks the same element as the host's slot-order loop in
@@ -315,10 +319,8 @@ __global__ void refit_nodes_kernel(RefitArgs a) {
 // axes' exponents with the same bvh8_exponent, each lane quantizes its own
 // slot with the same bvh8_quantize, and the bytes are
 // packed into words with shuffles and stored as four 16-byte words.
-__global__ void __launch_bounds__(128) refit_bvh8_kernel(RefitArgs a) {
-    if (a.state[kWordBad])
-        return;
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void refit_bvh8(const RefitArgs& a, uint32_t block) {
+    const uint64_t t = (uint64_t)block * kGridBlock + threadIdx.x;
     const uint64_t node = t >> 3;
     const uint32_t slot = (uint32_t)(t & 7u);
     const bool live = node < a.n8;  // the same for the eight lanes of a node
@@ -394,6 +396,20 @@ __global__ void __launch_bounds__(128) refit_bvh8_kernel(RefitArgs a) {
     out[slot] = v;
 }
 
+// Pass 4 in one launch: the grid nodes' blocks, then the BVH8 nodes', which
+// read different layouts and wait for nothing but pass 3.  As two kernels they
+// cost a frame of a refit and its rays over BVH8 109 us at 5,000 triangles and
+// 743 at 1M; in one launch 102 and 726.
+__global__ void __launch_bounds__(kGridBlock) refit_quantize_kernel(RefitArgs a) {
+    if (a.state[kWordBad])
+        return;
+    if (blockIdx.x < a.grid_blocks)
+        write_grid<true>(static_cast<const igxrt_bvh4_node*>(a.nodes4), a.n4, a.prims, a.grid_nodes, a.grid, a.state,
+                         blockIdx.x, a.grid_blocks);
+    else
+        refit_bvh8(a, blockIdx.x - a.grid_blocks);
+}
+
 }  // namespace
 
 extern "C" {
@@ -459,9 +475,13 @@ igxrt_status igxrt_scene_refit(igxrt_context* ctx, igxrt_scene* scene, const igx
     const uint32_t nodes = a.n2 + a.n4;
     if (nodes)
         refit_nodes_kernel<<<(nodes + 127) / 128, 128, 0, s>>>(a);
-    if (a.n8)
-        refit_bvh8_kernel<<<(uint32_t)((8 * (uint64_t)a.n8 + 127) / 128), 128, 0, s>>>(a);
-    e = write_grid_nodes(ctx, scene, true, s);
+    a.grid_nodes = scene->grid_nodes;
+    a.grid = scene->grid;
+    a.grid_blocks = scene->grid_fits ? grid_write_blocks(ctx, a.n4) : 0;
+    const uint32_t blocks8 = (uint32_t)((8 * (uint64_t)a.n8 + kGridBlock - 1) / kGridBlock);
+    if (a.grid_blocks + blocks8)
+        refit_quantize_kernel<<<a.grid_blocks + blocks8, kGridBlock, 0, s>>>(a);
+    e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "refit launch");
     uint32_t w[kRefitStateWords];
