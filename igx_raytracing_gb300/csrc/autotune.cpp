@@ -8,7 +8,9 @@
 // caller's items (median of `reps` repetitions after one warm-up), as one
 // batched launch or, with IGXRT_TUNE_PLAIN, as one plain launch per item.
 // Results can be cached in a text file, one line per (GPU name, class key):
-//     <gpu>|<key>\t<block> <stack> <packet> <layout> <ctas> <refill> <phase_break>\t<ms>
+//     <gpu>|<nodes>|<key>\t<block> <stack> <packet> <layout> <ctas> <refill> <phase_break>\t<ms>
+// <nodes> names what the launches trace (kNodes), so that entries timed on
+// other kernels are not taken for these.
 // The default class key buckets the workload by item count, total rays,
 // total triangles (powers of two) and the share of any-hit items.
 #include <cuda_runtime.h>
@@ -27,6 +29,8 @@
 using namespace igxrt;
 
 namespace {
+
+constexpr const char* kNodes = "grid";
 
 int log2_bucket(uint64_t x) {
     int b = 0;
@@ -224,7 +228,7 @@ extern "C" igxrt_status igxrt_autotune(igxrt_context* ctx, const igxrt_batch_ite
                 mask &= ~(1u << l);
     if (!(mask & ((1u << IGXRT_LAYOUT_COUNT) - 1)))
         return fail(ctx, IGXRT_ERROR_UNSUPPORTED, "autotune: no node layout common to all scenes");
-    const std::string key = ctx->device_name + "|" +
+    const std::string key = ctx->device_name + "|" + kNodes + "|" +
                             ((opts && opts->class_key) ? std::string(opts->class_key) : derive_key(items, count)) +
                             (plain ? "|plain" : "");
     const char* cache = opts ? opts->cache_path : nullptr;
@@ -259,6 +263,15 @@ extern "C" igxrt_status igxrt_autotune(igxrt_context* ctx, const igxrt_batch_ite
                 cur.layout = l;
                 break;
             }
+    // BVH2 and BVH4 name the same launch where every scene has grid nodes: one
+    // of them is timed, and the name the search starts from stays
+    bool grid = true;
+    for (uint32_t i = 0; i < count; ++i)
+        grid = grid && items[i].scene && grid_or_empty(*items[i].scene, IGXRT_LAYOUT_BVH2) &&
+               grid_or_empty(*items[i].scene, IGXRT_LAYOUT_BVH4);
+    const auto same_nodes = [grid](uint32_t a, uint32_t b) {
+        return grid && a != IGXRT_LAYOUT_BVH8 && b != IGXRT_LAYOUT_BVH8;
+    };
     float cur_ms = t.time(cur);
     if (cur_ms < 0)
         return fail(ctx, IGXRT_ERROR_CUDA, "autotune: the starting parameters do not launch");
@@ -272,6 +285,7 @@ extern "C" igxrt_status igxrt_autotune(igxrt_context* ctx, const igxrt_batch_ite
     for (int round = 0; round < 2; ++round) {
         bool changed = false;
         for (int dim = 0; dim < 6; ++dim) {
+            uint32_t timed = cur.layout;  // dim 0: the candidate before
             const std::vector<uint32_t>& vals = dim == 0   ? layouts
                                                 : dim == 1 ? packets
                                                 : dim == 2 ? refills
@@ -285,8 +299,11 @@ extern "C" igxrt_status igxrt_autotune(igxrt_context* ctx, const igxrt_batch_ite
                                   : dim == 4 ? &c.stack_depth : &c.phase_break;
                 if (*field == v)
                     continue;
-                if (dim == 0 && !((mask >> v) & 1u))
-                    continue;
+                if (dim == 0) {
+                    if (!((mask >> v) & 1u) || same_nodes(v, cur.layout) || same_nodes(v, timed))
+                        continue;
+                    timed = v;
+                }
                 *field = v;
                 const float ms = t.time(c);
                 if (ms > 0 && ms < cur_ms * 0.99f) {
