@@ -80,21 +80,20 @@ __device__ __forceinline__ void finish_ray(const KernelArgs& a, uint32_t i, cons
 // mixed scene's closest-hit kernel until there is one for every lane: the uv
 // takes binary64 asin and atan, and with a lane or two of a warp at a time
 // they kept that pipe half busy on 1M rays of which 15% hit a sphere (664 us;
-// 615 in batches; 602 with no uv at all).  In shared memory, per warp: the
-// number of entries, then {ray, record, t} each; fewer than 32 are left after
-// a flush and a round adds at most one per lane.
-constexpr uint32_t kUvEntries = 64, kUvWords = 4 + 3 * kUvEntries;
+// 615 in batches; 602 with no uv at all, at 64 registers).  In shared memory, per warp: the
+// number of entries, then {ray, object, t, sphere_offset} each, so that no ray
+// is read twice (over host arrays in place that is the link); fewer than 32 are left
+// after a flush and a round adds at most one per lane.
+constexpr uint32_t kUvEntries = 64, kUvEntryWords = 6, kUvWords = 4 + kUvEntryWords * kUvEntries;
 
 __device__ __forceinline__ void flush_uv(const KernelArgs& a, uint32_t* batch, uint32_t take, uint32_t lane) {
     const uint32_t base = batch[0] - take;
     if (lane < take) {
-        const uint32_t* e = batch + 4 + 3 * (base + lane);
-        const RayState r = load_ray(a.rays, e[0], 0u);
-        const float4 c = __ldg(a.prims + 3 * (size_t)e[1]);
-        const float t = __uint_as_float(e[2]);
+        const uint32_t* e = batch + 4 + kUvEntryWords * (base + lane);
         float u, v;
-        sphere_uv(r, c.x, c.y, c.z, t, u, v);
-        __stcs(reinterpret_cast<float4*>(a.hits) + e[0], make_float4(t, u, v, c.w));  // c.w: the object
+        sphere_uv(__uint_as_float(e[3]), __uint_as_float(e[4]), __uint_as_float(e[5]), u, v);
+        __stcs(reinterpret_cast<float4*>(a.hits) + e[0],
+               make_float4(__uint_as_float(e[2]), u, v, __uint_as_float(e[1])));
     }
     __syncwarp();
     if (lane == 0)
@@ -174,10 +173,16 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
     uint32_t link = lane;
     const auto write_ray = [&](bool occluded) {
         if (UV_BATCH && __float_as_uint(best.v) == kUvPending) {
-            uint32_t* e = uv + 4 + 3 * atomicAdd(uv, 1u);
+            const float4 c = __ldg(a.prims + 3 * (size_t)__float_as_uint(best.u));
+            uint32_t* e = uv + 4 + kUvEntryWords * atomicAdd(uv, 1u);
+            float nx, ny, nz;
+            sphere_offset(r, c.x, c.y, c.z, best.t, nx, ny, nz);
             e[0] = ray;
-            e[1] = __float_as_uint(best.u);
+            e[1] = __float_as_uint(c.w);
             e[2] = __float_as_uint(best.t);
+            e[3] = __float_as_uint(nx);
+            e[4] = __float_as_uint(ny);
+            e[5] = __float_as_uint(nz);
         } else {
             finish_ray<ANY, COUNT, MIXED>(a, ray, r, best, occluded, nf, pf);
         }

@@ -585,18 +585,22 @@ __device__ __forceinline__ bool sphere_hit(const RayState& r, float cx, float cy
     return !(Q2 > R2);
 }
 
-// The sphere's uv (primitive.glsl:189-204).  asin and atan give the
-// correctly rounded binary32 value: evaluated in binary64 (CUDA's asin /
+// The centre seen from the hit point (primitive.glsl:189-204, its first lines).
+__device__ __forceinline__ void sphere_offset(const RayState& r, float cx, float cy, float cz, float hitT, float& nx,
+                                              float& ny, float& nz) {
+    const float ox = __fadd_rn(__fmul_rn(hitT, r.dx), r.ox), oy = __fadd_rn(__fmul_rn(hitT, r.dy), r.oy),
+                oz = __fadd_rn(__fmul_rn(hitT, r.dz), r.oz);
+    nx = __fsub_rn(cx, ox), ny = __fsub_rn(cy, oy), nz = __fsub_rn(cz, oz);
+}
+
+// The sphere's uv (the rest of primitive.glsl:189-204) from sphere_offset.
+// asin and atan give the correctly rounded binary32 value: evaluated in binary64 (CUDA's asin /
 // atan, a few binary64 ulp) and rounded once, which lands on the correctly
 // rounded float unless the binary64 value falls within its error of a
 // binary32 rounding midpoint.  The oracle evaluates them the same way, so u
 // and v, which cancel towards 0 near the poles and the seam (lat * 1/pi +
 // 0.5), come out bit for bit instead of many float ulp apart.
-__device__ __forceinline__ void sphere_uv(const RayState& r, float cx, float cy, float cz, float hitT,
-                                          float& u, float& v) {
-    const float ox = __fadd_rn(__fmul_rn(hitT, r.dx), r.ox), oy = __fadd_rn(__fmul_rn(hitT, r.dy), r.oy),
-                oz = __fadd_rn(__fmul_rn(hitT, r.dz), r.oz);
-    const float nx = __fsub_rn(cx, ox), ny = __fsub_rn(cy, oy), nz = __fsub_rn(cz, oz);
+__device__ __forceinline__ void sphere_uv(float nx, float ny, float nz, float& u, float& v) {
     const float len = __fsqrt_rn(dot3f(nx, ny, nz, nx, ny, nz));
     const float ux = __fdiv_rn(nx, len), uy = __fdiv_rn(ny, len), uz = __fdiv_rn(nz, len);
     const float lat = __double2float_rn(asin((double)uz));
@@ -669,7 +673,9 @@ __device__ __forceinline__ void finish_uv(const float4* __restrict__ prims, cons
     if (__float_as_uint(best.v) != kUvPending)
         return;
     const float4 c = __ldg(prims + 3 * (size_t)__float_as_uint(best.u));
-    sphere_uv(r, c.x, c.y, c.z, best.t, best.u, best.v);
+    float nx, ny, nz;
+    sphere_offset(r, c.x, c.y, c.z, best.t, nx, ny, nz);
+    sphere_uv(nx, ny, nz, best.u, best.v);
 }
 
 // Record `i` of a mixed scene against the ray.  Returns true when an any-hit
