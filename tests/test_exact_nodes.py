@@ -141,3 +141,80 @@ def test_a_captured_trace_over_a_range_that_overflows(ctx):
         for f in ("prim", "t", "u", "v"):
             assert np.array_equal(got[f][ok].view(np.uint32), expect[f][ok].view(np.uint32)), f
     scene.close()
+
+
+@pytest.mark.parametrize("layout", [0, 1])
+def test_a_batch_with_one_scene_off_the_grid(ctx, layout):
+    """One launch traces one kind of nodes: a scene without usable grid nodes
+    takes the batch to the exact ones, triangles and mixed, both query modes."""
+    import torch
+
+    sets = [scenes.random_triangles(n, 8120 + n, mu=math.log(0.04)) for n in (2000, 900, 3000)]
+    sets[1] = _far(sets[1])
+    live = [ctx.create_scene(t) for t in sets]
+    assert [uses_grid(s) for s in live] == [True, False, True]
+    rays = scenes.incoherent_rays(3000, 8121)
+    d_rays = _device(rays)
+    items, expect = [], []
+    for s, t in zip(live, sets):
+        for mode in (0, 1):
+            out = (torch.full((len(rays),), 9, dtype=torch.int32, device="cuda") if mode
+                   else torch.full((len(rays), 4), -1.0, device="cuda"))
+            items.append((s, d_rays, None, out, mode))
+            expect.append((pyoracle.trace_occlusion if mode else pyoracle.trace_geometry)(t, rays))
+    batch = ctx.create_batch(items, params={"layout": layout})
+    for launch in (batch.launch, lambda: ctx.trace_batch(items)):
+        launch()
+        torch.cuda.synchronize()
+        for (_, _, _, out, mode), (want, flags) in zip(items, expect):
+            ok = flags == 0
+            if mode:
+                assert np.array_equal(out.cpu().numpy().view(np.uint32)[ok], want[ok])
+                out.fill_(9)
+            else:
+                got = out.cpu().numpy().view(HIT_DTYPE).reshape(-1)
+                for f in ("prim", "t", "u", "v"):
+                    assert np.array_equal(got[f][ok].view(np.uint32), want[f][ok].view(np.uint32)), f
+                out.fill_(-1)
+    assert not igx.lib().igxrt_internal_batch_uses_grid(batch._h)
+    batch.close()
+    for s in live:
+        s.close()
+
+
+def test_a_served_batch_with_one_scene_off_the_grid(ctx):
+    """The server's table is rewritten for the exact nodes when a request over
+    such a scene joins the batch, whatever was in it before."""
+    sets = [scenes.random_triangles(n, 8130 + n, mu=math.log(0.04)) for n in (1500, 800)]
+    sets[1] = _far(sets[1])
+    live = [ctx.create_scene(t) for t in sets]
+    assert [uses_grid(s) for s in live] == [True, False]
+    srv = igx.Server(ctx, streams=1, slice_rays=700)
+    ids = [srv.add_scene(s) for s in live]
+    requests = []
+    for k in range(24):  # fit ones first, so that a table is half filled
+        which = 1 if k % 6 == 5 else 0
+        rays = scenes.incoherent_rays(400 + 100 * k, 8140 + k)
+        prev = np.where(np.arange(len(rays)) % 3 == 0, k, 0xFFFFFFFF).astype(np.uint32) if k % 2 else None
+        requests.append((which, rays, prev, k % 3 == 2))
+    tickets = [srv.submit(ids[w], r, p, int(m)) for w, r, p, m in requests]
+    for t, (w, rays, prev, mode) in zip(tickets, requests):
+        got = srv.wait(t)["out"]
+        want, flags = (pyoracle.trace_occlusion if mode else pyoracle.trace_geometry)(sets[w], rays, prev)
+        ok = flags == 0
+        if mode:
+            assert np.array_equal(got[ok], want[ok])
+        else:
+            for f in ("prim", "t", "u", "v"):
+                assert np.array_equal(got[f][ok].view(np.uint32), want[f][ok].view(np.uint32)), f
+    srv.close()
+    for s in live:
+        s.close()
+
+
+@pytest.mark.parametrize("leaf", [1, 4, 16])
+def test_ordinary_scenes_are_on_the_grid(ctx, leaf):
+    for tris in (scenes.displaced_sphere(64, 32), scenes.random_triangles(4000, 8150), scenes.heightfield(40, 30, 8151)):
+        scene = ctx.create_scene(tris, max_leaf_size=leaf)
+        assert uses_grid(scene)
+        scene.close()
