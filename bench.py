@@ -54,6 +54,7 @@ rank traces the whole step on its own GPU (weak scaling).
 from __future__ import annotations
 
 import argparse
+import ctypes as C
 import hashlib
 import json
 import math
@@ -74,8 +75,9 @@ RAY_BYTES = 32
 HIT_BYTES = 16
 OCC_BYTES = 4
 PREV_BYTES = 4
-NODE_BYTES = {0: 64, 1: 128, 2: 96}
-LAYOUT_NAMES = {0: "bvh2", 1: "bvh4", 2: "bvh8"}
+GRID = 3  # the nodes that launches over BVH2 and BVH4 trace where the scene has them
+NODE_BYTES = {0: 64, 1: 128, 2: 96, GRID: 64}
+LAYOUT_NAMES = {0: "bvh2", 1: "bvh4", 2: "bvh8", GRID: "grid"}
 LAYOUT_IDS = {v: k for k, v in LAYOUT_NAMES.items()}
 PRIM_BYTES = 48
 
@@ -141,6 +143,31 @@ def algorithmic_bytes(nf: np.ndarray, pf: np.ndarray, mode: int, has_prev: bool,
     per_ray = RAY_BYTES + (HIT_BYTES if mode == 0 else OCC_BYTES) + (PREV_BYTES if has_prev else 0)
     return int(per_ray * len(nf) + NODE_BYTES[layout] * int(nf.sum(dtype=np.int64))
                + PRIM_BYTES * int(pf.sum(dtype=np.int64)))
+
+
+def traced_nodes(scene, layout: int) -> int:
+    """The nodes that a launch over the scene naming `layout` traces."""
+    import igx_raytracing_gb300 as igx
+
+    return GRID if layout != 2 and igx.lib().igxrt_internal_uses_grid(scene.handle) else layout
+
+
+def count_fetches(ctx, scene, rays, prev, mode: int, nodes: int):
+    """Node and primitive records that the launch over `nodes` (traced_nodes)
+    fetches per ray, from that kernel's instrumented twin."""
+    if nodes != GRID:
+        return ctx.count_fetches(scene, rays, prev, mode=mode, layout=nodes)
+    import igx_raytracing_gb300 as igx
+    from igx_raytracing_gb300._capi import check
+
+    rays = igx.as_rays(rays)
+    nf, pf = np.zeros(len(rays), np.uint32), np.zeros(len(rays), np.uint32)
+    prev = None if prev is None else np.ascontiguousarray(prev, np.uint32)
+    ptr = lambda a: C.c_void_p(a.ctypes.data if a is not None else None)
+    check(igx.lib().igxrt_internal_count_grid_fetches(ctx.handle, scene.handle, ptr(rays), ptr(prev),
+                                                      C.c_uint32(len(rays)), C.c_uint32(mode), ptr(nf), ptr(pf)),
+          ctx.handle, "count_grid_fetches")
+    return nf, pf
 
 
 def measured_peaks() -> dict:
@@ -566,11 +593,12 @@ def measure_plain(args, ctx, dev, name: str, world: int, lite: bool = False) -> 
     peaks = measured_peaks()
     per_batch = []
     for i, (bname, rays, prev, mode) in enumerate(batches):
-        nf, pf = ctx.count_fetches(scene, rays, prev, mode=mode, layout=layouts[i])
-        b = algorithmic_bytes(nf, pf, mode, prev is not None, layouts[i])
+        nodes = traced_nodes(scene, layouts[i])
+        nf, pf = count_fetches(ctx, scene, rays, prev, mode, nodes)
+        b = algorithmic_bytes(nf, pf, mode, prev is not None, nodes)
         ms = float(launch_ms[:, i].mean())
         per_batch.append({"batch": bname, "rays": len(rays), "mode": "any" if mode else "closest",
-                          "layout": LAYOUT_NAMES[layouts[i]],
+                          "layout": LAYOUT_NAMES[layouts[i]], "nodes": LAYOUT_NAMES[nodes],
                           "ms": round(ms, 4), "bytes": b, "nodes_per_ray": round(float(nf.mean()), 3),
                           "prims_per_ray": round(float(pf.mean()), 3),
                           "gbs": round(b / (ms / 1e3) / 1e9, 1),
@@ -580,7 +608,7 @@ def measure_plain(args, ctx, dev, name: str, world: int, lite: bool = False) -> 
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"],
                 "unit": "GB/s", "frac": round(achieved / peaks["hbm_gbs"], 4),
                 "traffic": traffic_from_profiles(cfg["workload"], dom["batch"], LAYOUT_IDS[dom["layout"]]),
-                "kernel": f"trace_kernel<{dom['layout']},{dom['mode']}> ({dom['batch']})",
+                "kernel": f"trace_kernel<{dom['nodes']},{dom['mode']}> ({dom['batch']})",
                 "peak_source": peaks["source"], "bytes_per_launch": dom["bytes"]}
     step_bytes = sum(b["bytes"] for b in per_batch)
 
@@ -810,10 +838,13 @@ def measure_batch(args, ctx, dev, world: int) -> dict:
     # roofline over the whole batch launch
     peaks = measured_peaks()
     layout = tuned["layout"]
+    # one launch traces one kind of nodes: the grid nodes if every scene has them
+    on_grid = all(traced_nodes(it[0], layout) == GRID for it in items)
+    nodes = GRID if on_grid else layout
     bytes_total = 0
     for (scene, _, _, _, _), rays in zip(items, host_rays):
-        nf, pf = ctx.count_fetches(scene, rays, None, mode=0, layout=layout)
-        bytes_total += algorithmic_bytes(nf, pf, 0, False, layout)
+        nf, pf = count_fetches(ctx, scene, rays, None, 0, nodes)
+        bytes_total += algorithmic_bytes(nf, pf, 0, False, nodes)
     achieved = bytes_total / (bat_ms / 1e3) / 1e9
 
     # e2e from pinned host memory: a batch whose items are the pinned arrays
@@ -855,7 +886,7 @@ def measure_batch(args, ctx, dev, world: int) -> dict:
            "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"],
                         "unit": "GB/s", "frac": round(achieved / peaks["hbm_gbs"], 4),
                         "traffic": traffic_from_profiles(wl, "batch", layout),
-                        "kernel": f"batch_kernel<{LAYOUT_NAMES[layout]}>", "peak_source": peaks["source"],
+                        "kernel": f"batch_kernel<{LAYOUT_NAMES[nodes]}>", "peak_source": peaks["source"],
                         "bytes_per_launch": int(bytes_total)},
            "e2e": {"value": round(world * total_rays / (e2e_ms / 1e3) / 1e6, 3), "unit": UNIT,
                    "h2d_bytes_per_step": total_rays * RAY_BYTES,
@@ -1182,11 +1213,12 @@ def run_pass_bench(args, rank: int, world: int, local_rank: int):
         ms = statistics.mean(_event_ms(torch, fused, args.steps, flush, stream))
         clk = clocks.stop()
         split_ms = statistics.mean(_event_ms(torch, split, args.steps, flush, stream))
-        nf, pf = ctx.count_fetches(scene, rays, None, mode=0, layout=layout)
+        nodes = traced_nodes(scene, layout)
+        nf, pf = count_fetches(ctx, scene, rays, None, 0, nodes)
         # per pixel: the trace's hit record written and read back by the
         # encoding kernel (16 + 16 B), dirObject written (16 B); on a hit also
         # uvNormal (16 B) and the hit triangle's normals (48 B); no ray is read
-        b = int(48 * len(rays) + (16 + 48) * int(hit.sum()) + NODE_BYTES[layout] * int(nf.sum(dtype=np.int64))
+        b = int(48 * len(rays) + (16 + 48) * int(hit.sum()) + NODE_BYTES[nodes] * int(nf.sum(dtype=np.int64))
                 + PRIM_BYTES * int(pf.sum(dtype=np.int64)))
         hdo = torch.empty((h, w, 4), dtype=torch.float32).pin_memory().numpy()
         huv = torch.zeros((h, w, 4), dtype=torch.float32).pin_memory().numpy()
@@ -1200,7 +1232,7 @@ def run_pass_bench(args, rank: int, world: int, local_rank: int):
         n = w * h
         line = _line(args, world, world * n / (ms / 1e3) / 1e6, ms,
                      dict(cfg, workload="gbuffer_sphere_1m_1080p", rays_per_step=n),
-                     roofline=_roofline(b, ms, f"trace_kernel<{LAYOUT_NAMES[layout]},closest,camera> + "
+                     roofline=_roofline(b, ms, f"trace_kernel<{LAYOUT_NAMES[nodes]},closest,camera> + "
                                                "gbuffer_encode_kernel",
                                         traffic_from_profiles("gbuffer_sphere_1m_1080p", "gbuffer", layout)),
                      e2e={"value": round(world * n / (e2e_ms / 1e3) / 1e6, 3), "unit": UNIT,
@@ -1246,11 +1278,12 @@ def run_pass_bench(args, rank: int, world: int, local_rank: int):
         ms = statistics.mean(_event_ms(torch, fused, args.steps, flush, stream))
         clk = clocks.stop()
         plain_ms = statistics.mean(_event_ms(torch, plain, args.steps, flush, stream))
-        nf, pf = ctx.count_fetches(scene, shadow, prev, mode=1, layout=layout)
+        nodes = traced_nodes(scene, layout)
+        nf, pf = count_fetches(ctx, scene, shadow, prev, 1, nodes)
         # per traced ray: ray (32 B) + its pixel's object (4 B, the prevHit);
         # every pixel's object word is read, every mask word written
         n = int(hit.sum())
-        b = int(32 * n + 4 * w * h + 4 * words + NODE_BYTES[layout] * int(nf.sum(dtype=np.int64))
+        b = int(32 * n + 4 * w * h + 4 * words + NODE_BYTES[nodes] * int(nf.sum(dtype=np.int64))
                 + PRIM_BYTES * int(pf.sum(dtype=np.int64)))
         # pinned host copies of the pass's inputs and mask
         h_pix = torch.from_numpy(pix_rays.view(np.float32).reshape(-1, 8).copy()).pin_memory().numpy()
@@ -1267,7 +1300,7 @@ def run_pass_bench(args, rank: int, world: int, local_rank: int):
         line = _line(args, world, world * n / (ms / 1e3) / 1e6, ms,
                      dict(cfg, workload="shadowmask_sphere_1m_1080p_1_sample", rays_per_step=n,
                           light=list(scenes.SPHERE_LIGHT)),
-                     roofline=_roofline(b, ms, f"shadow pass: compact + trace_kernel<{LAYOUT_NAMES[layout]},any> + pack",
+                     roofline=_roofline(b, ms, f"shadow pass: compact + trace_kernel<{LAYOUT_NAMES[nodes]},any> + pack",
                                         traffic_from_profiles("shadowmask_sphere_1m_1080p_1_sample", "pass", layout)),
                      e2e={"value": round(world * n / (e2e_ms / 1e3) / 1e6, 3), "unit": UNIT,
                           "h2d_bytes_per_step": 36 * w * h, "d2h_bytes_per_step": 4 * words,
@@ -1321,9 +1354,10 @@ def run_mixed_bench(args, rank: int, world: int, local_rank: int):
     clocks.start()
     ms = statistics.mean(_event_ms(torch, fn, args.steps, flush, stream))
     clk = clocks.stop()
-    nf, pf = ctx.count_fetches(scene, rays, None, mode=0, layout=layout)
+    nodes = traced_nodes(scene, layout)
+    nf, pf = count_fetches(ctx, scene, rays, None, 0, nodes)
     planes = len(sc["planes"])
-    b = algorithmic_bytes(nf, pf, 0, False, layout) + 16 * planes * len(rays)
+    b = algorithmic_bytes(nf, pf, 0, False, nodes) + 16 * planes * len(rays)
     hrays = torch.from_numpy(rays.view(np.float32).reshape(-1, 8).copy()).pin_memory().numpy().view(igx.RAY_DTYPE).reshape(-1)
     hout = torch.empty((len(rays), 4), dtype=torch.float32).pin_memory().numpy().view(igx.HIT_DTYPE).reshape(-1)
     ctx.trace_closest(scene, hrays, out=hout)
@@ -1340,7 +1374,7 @@ def run_mixed_bench(args, rank: int, world: int, local_rank: int):
            "launch": ctx.launch_params, "launch_chosen_by": tuned_by, "bvh_build_s": round(build_s, 2),
            "l2": "256 MiB buffer written between timed steps"}
     line = _line(args, world, world * n / (ms / 1e3) / 1e6, ms, cfg,
-                 roofline=_roofline(b, ms, f"trace_kernel<{LAYOUT_NAMES[layout]},closest,mixed>",
+                 roofline=_roofline(b, ms, f"trace_kernel<{LAYOUT_NAMES[nodes]},closest,mixed>",
                                     traffic_from_profiles(cfg["workload"], "mixed", layout)),
                  e2e={"value": round(world * n / (e2e_ms / 1e3) / 1e6, 3), "unit": UNIT,
                       "h2d_bytes_per_step": 32 * n, "d2h_bytes_per_step": 16 * n,
@@ -1447,19 +1481,19 @@ def run_dynamic_bench(args, rank: int, world: int, local_rank: int):
     e2e_ms = max_over_ranks(1000 * statistics.mean(e2e_s), dev)
     e2e_spread = (round(1000 * min(e2e_s), 3), round(1000 * max(e2e_s), 3))
 
-    nf, pf = ctx.count_fetches(scene, rays, None, mode=0, layout=layout)
+    nodes = traced_nodes(scene, layout)
+    nf, pf = count_fetches(ctx, scene, rays, None, 0, nodes)
     n = len(rays)
-    b = algorithmic_bytes(nf, pf, 0, False, layout)
-    # a frame: the refit's scan, records, nodes, BVH8 and grid passes, then the trace
+    b = algorithmic_bytes(nf, pf, 0, False, nodes)
+    # a frame: the refit's scan, records, nodes and quantizing passes, then the trace
     si = scene.info
-    refit_launches = (2 + (si["bvh2_nodes"] + si["bvh4_nodes"] > 0) + (si["bvh8_nodes"] > 0)
-                      + (si["bvh4_nodes"] > 0) + 1)
+    refit_launches = 2 + 2 * (si["bvh2_nodes"] + si["bvh4_nodes"] > 0) + 1
     cfg = {"workload": "dynamic_sphere_1m_refit_1080p_primary", "triangles": len(tris),
            "rays_per_step": n, "layout": LAYOUT_NAMES[layout], "launch": ctx.launch_params,
            "frames": len(frames), "host_sah_build_s": round(host_build_s, 3),
            "l2": "256 MiB buffer written between timed steps"}
     line = _line(args, world, world * n / (ms / 1e3) / 1e6, ms, cfg,
-                 roofline=_roofline(b, trace_only, f"trace_kernel<{LAYOUT_NAMES[layout]},closest> (frame rays)",
+                 roofline=_roofline(b, trace_only, f"trace_kernel<{LAYOUT_NAMES[nodes]},closest> (frame rays)",
                                     traffic_from_profiles(cfg["workload"], "frame", layout)),
                  frame={"refit_ms": round(refit_only, 4), "trace_ms": round(trace_only, 4),
                         "refit_plus_trace_ms": round(ms, 4),

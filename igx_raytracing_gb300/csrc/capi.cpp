@@ -717,6 +717,52 @@ igxrt_status igxrt_count_fetches(igxrt_context* ctx, const igxrt_scene* scene, c
     return st;
 }
 
+igxrt_status igxrt_internal_count_grid_fetches(igxrt_context* ctx, const igxrt_scene* scene, const igxrt_ray* rays,
+                                               const uint32_t* prev_hit, uint32_t count, uint32_t mode,
+                                               uint32_t* node_fetches, uint32_t* prim_fetches) {
+    if (!ctx)
+        return IGXRT_ERROR_INVALID_ARGUMENT;
+    igxrt_status st = check_scene(ctx, scene);
+    if (st != IGXRT_OK)
+        return st;
+    if (mode > 1 || !rays || !node_fetches || !prim_fetches || !use_grid(*scene, IGXRT_LAYOUT_BVH2))
+        return fail(ctx, IGXRT_ERROR_INVALID_ARGUMENT, "mode 0/1, rays, both count arrays and a scene on the grid");
+    if (count == 0)
+        return IGXRT_OK;
+    DeviceGuard guard(ctx->device);
+    // [rays][prev][results][node counts][record counts]
+    const size_t rb = round_up((size_t)count * sizeof(igxrt_ray), 256), wb = round_up((size_t)count * 4, 256);
+    const size_t ob = round_up((size_t)count * sizeof(igxrt_hit), 256);
+    char* mem = nullptr;
+    cudaError_t e = cudaMalloc(&mem, rb + ob + 3 * wb);
+    if (e != cudaSuccess)
+        return cuda_fail(ctx, e, "count scratch");
+    uint32_t* prev = reinterpret_cast<uint32_t*>(mem + rb);
+    char* out = mem + rb + wb;
+    uint32_t* nf = reinterpret_cast<uint32_t*>(out + ob);
+    uint32_t* pf = reinterpret_cast<uint32_t*>(out + ob + wb);
+    e = cudaMemcpy(mem, rays, (size_t)count * sizeof(igxrt_ray), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && prev_hit)
+        e = cudaMemcpy(prev, prev_hit, (size_t)count * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        TraceRequest req{scene, reinterpret_cast<igxrt_ray*>(mem), prev_hit ? prev : nullptr, count, mode,
+                         mode == 0 ? reinterpret_cast<igxrt_hit*>(out) : nullptr,
+                         mode == 1 ? reinterpret_cast<uint32_t*>(out) : nullptr, nf, pf};
+        req.grid_fetches = true;
+        igxrt_launch_params p = ctx->params;
+        p.layout = IGXRT_LAYOUT_BVH2;
+        st = launch_trace(ctx, req, p, nullptr);
+    }
+    if (e == cudaSuccess && st == IGXRT_OK)
+        e = cudaMemcpy(node_fetches, nf, (size_t)count * 4, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && st == IGXRT_OK)
+        e = cudaMemcpy(prim_fetches, pf, (size_t)count * 4, cudaMemcpyDeviceToHost);
+    cudaFree(mem);
+    if (st == IGXRT_OK && e != cudaSuccess)
+        st = cuda_fail(ctx, e, "grid fetch counts");
+    return st == IGXRT_OK ? read_status(ctx) : st;
+}
+
 igxrt_status igxrt_fetch_hits(igxrt_context* ctx, const igxrt_hit* device_hits, uint32_t count,
                               igxrt_hit* host_hits, void* stream) {
     if (!ctx || (count && (!device_hits || !host_hits)))

@@ -179,6 +179,9 @@ struct TraceRequest {
     // non-null: the rays are this camera's, one per pixel (closest hit on a
     // triangle scene; `rays` and `prev` unused)
     const CameraSource* camera = nullptr;
+    // instrumented launches: over the grid nodes (the scene must use them)
+    // instead of the named layout's
+    bool grid_fetches = false;
 };
 
 // Records `msg` as the context's last error and returns `st`.
@@ -289,13 +292,17 @@ class DeviceGuard {
 
 }  // namespace igxrt
 
-// Entry points for the tests, in no public header: which nodes the scene's
+// Entry points for the tests and the benchmark, in no public header: which nodes the scene's
 // BVH2 and BVH4 launches trace now (1: grid nodes, 0: exact), and a context's
 // limit on the records of a scene with grid nodes, for scenes created after
 // the call (0: every scene stays on the exact nodes for its life).
 extern "C" {
 uint32_t igxrt_internal_uses_grid(const igxrt_scene* scene);
 void igxrt_internal_set_grid_records(igxrt_context* ctx, uint64_t records);
+// igxrt_count_fetches for the launches that trace grid nodes (host arrays).
+igxrt_status igxrt_internal_count_grid_fetches(igxrt_context* ctx, const igxrt_scene* scene, const igxrt_ray* rays,
+                                               const uint32_t* prev_hit, uint32_t count, uint32_t mode,
+                                               uint32_t* node_fetches, uint32_t* prim_fetches);
 // The nodes of a batch's latest launch (1: grid nodes).
 uint32_t igxrt_internal_batch_uses_grid(const igxrt_batch* batch);
 }

@@ -268,6 +268,8 @@ __global__ void __maxnreg__(trace_kernel_regs(LAYOUT, ANY, MIXED)) trace_kernel(
         bool overflow = false;
         node_phase<LAYOUT, COUNT, MIXED>(a.nodes, working, wmask, a.phase_break, next, r, best, st, overflow, nf,
                                             WARP_LEAVES && a.phase_break < 32u ? kLeafLanes : 33u);
+        if (COUNT && GRID && working && next < 0)
+            pf += ((uint32_t)next & 15u) + 1u;  // the leaf's records
         bool leaf_occluded = false;
         if constexpr (WARP_LEAVES)
             warp_leaf_phase<ANY>(a.prims, working, lane, lower, leaves, next, r.prev, best, st, leaf_occluded);
@@ -349,12 +351,16 @@ static KernelFn select_kernel(uint32_t layout, bool any, bool count, bool mixed)
     return any ? trace_kernel<B2, true, false, false> : trace_kernel<B2, false, false, false>;
 }
 
-// The kernels over grid nodes (never instrumented: fetch counts describe the
-// exact layouts).
-static KernelFn select_grid_kernel(bool any, bool mixed, bool camera) {
+// The kernels over grid nodes; their instrumented twins count what the
+// benchmark's bytes are made of.
+static KernelFn select_grid_kernel(bool any, bool count, bool mixed, bool camera) {
     constexpr int G = (int)kLayoutGrid;
     if (camera)
         return trace_kernel<G, false, false, false, true>;
+    if (count && mixed)
+        return any ? trace_kernel<G, true, true, true> : trace_kernel<G, false, true, true>;
+    if (count)
+        return any ? trace_kernel<G, true, true, false> : trace_kernel<G, false, true, false>;
     if (mixed)
         return any ? trace_kernel<G, true, false, true> : trace_kernel<G, false, false, true>;
     return any ? trace_kernel<G, true, false, false> : trace_kernel<G, false, false, false>;
@@ -385,8 +391,9 @@ igxrt_status prepare_trace(igxrt_context* ctx, const TraceRequest& req, const ig
     const igxrt_scene* s = req.scene;
     if (req.camera && (s->mixed || req.mode != 0 || req.node_fetches))
         return fail(ctx, IGXRT_ERROR_UNSUPPORTED, "camera rays are traced for closest hits on triangles");
-    const bool grid = use_grid(*s, p.layout) && !req.node_fetches;
-    l.fn = grid         ? select_grid_kernel(req.mode == 1, s->mixed, req.camera != nullptr)
+    const bool grid = use_grid(*s, p.layout) && (!req.node_fetches || req.grid_fetches);
+    l.fn = grid         ? select_grid_kernel(req.mode == 1, req.node_fetches != nullptr, s->mixed,
+                                             req.camera != nullptr)
            : req.camera ? select_camera_kernel(p.layout)
                         : select_kernel(p.layout, req.mode == 1, req.node_fetches != nullptr, s->mixed);
     l.smem = (size_t)p.stack_depth * p.block_size * kStackEntryBytes +

@@ -289,10 +289,13 @@ __device__ __forceinline__ void node_phase(const float4* __restrict__ nodes, boo
         if ((uint32_t)__popc(dm) * phase_break <= waiting || waiting >= enough)
             break;
         if (down) {
-            if constexpr (LAYOUT == (int)kLayoutGrid)
+            if constexpr (LAYOUT == (int)kLayoutGrid) {
+                if (COUNT)
+                    ++nf;
                 next = visit_grid<MIXED>(nodes, next, r, best.tcull, st, overflow);
-            else
+            } else {
                 next = visit_node<LAYOUT, COUNT, MIXED>(nodes, next, r, best, st, overflow, nf);
+            }
         }
     }
 }
