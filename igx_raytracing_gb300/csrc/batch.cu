@@ -450,7 +450,7 @@ igxrt_status capture_form(igxrt_batch* b) {
         return st;
     BatchForm& f = b->forms[layout == kLayoutGrid ? 1 : 0];
     const size_t tb = (table.size() * sizeof(BatchItemDev) + 255) / 256 * 256;
-    cudaError_t e = cudaMalloc(&f.d_mem, tb + 256);
+    cudaError_t e = device_alloc(ctx, &f.d_mem, tb + 256);
     if (e == cudaSuccess && !table.empty())
         e = cudaMemcpy(f.d_mem, table.data(), table.size() * sizeof(BatchItemDev), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {

@@ -87,12 +87,23 @@ MemoryPool::~MemoryPool() {
     cudaMemPoolDestroy(pool);
 }
 
+cudaError_t device_alloc(igxrt_context* ctx, void** ptr, size_t bytes) {
+    cudaError_t e = cudaMalloc(ptr, bytes);
+    if (e == cudaErrorMemoryAllocation && ctx->pool) {
+        cudaGetLastError();
+        cudaDeviceSynchronize();  // frees queued into the pool
+        cudaMemPoolTrimTo(ctx->pool->pool, 0);
+        e = cudaMalloc(ptr, bytes);
+    }
+    return e;
+}
+
 cudaError_t pool_alloc(igxrt_context* ctx, void** ptr, size_t bytes, cudaStream_t stream, bool& pooled) {
     pooled = ctx->pool && cudaMallocFromPoolAsync(ptr, bytes, ctx->pool->pool, stream) == cudaSuccess;
     if (pooled)
         return cudaSuccess;
     cudaGetLastError();
-    return cudaMalloc(ptr, bytes);
+    return device_alloc(ctx, ptr, bytes);
 }
 
 // One device allocation per scene, 256-byte aligned sub-buffers in this
@@ -124,7 +135,8 @@ igxrt_status allocate_scene(igxrt_context* ctx, const igxrt_bvh_info& info, uint
     const size_t og = o8 + b8 + bs8, bg = s->grid_fits ? (size_t)n4 * 4 * sizeof(float4) : 0;
     const size_t bytes = og + bg + 2 * sizeof(float4);
     bool pooled = false;
-    cudaError_t e = pool ? pool_alloc(ctx, &s->d_mem, bytes, stream, pooled) : cudaMalloc(&s->d_mem, bytes);
+    cudaError_t e = pool ? pool_alloc(ctx, &s->d_mem, bytes, stream, pooled)
+                         : device_alloc(ctx, &s->d_mem, bytes);
     if (pooled)
         s->pool = ctx->pool;
     if (e != cudaSuccess) {
@@ -226,7 +238,7 @@ igxrt_status igxrt::grow_stage(igxrt_context* ctx, size_t bytes) {
     cudaError_t e = cudaMalloc(&ctx->d_stage, want);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        e = cudaMalloc(&ctx->d_stage, bytes);
+        e = device_alloc(ctx, &ctx->d_stage, bytes);
         want = bytes;
     }
     if (e != cudaSuccess)
@@ -707,7 +719,7 @@ igxrt_status igxrt_count_fetches(igxrt_context* ctx, const igxrt_scene* scene, c
                             IGXRT_TRACE_HOST_MEMORY, stream, node_fetches, prim_fetches, p);
     }
     void* d_out = nullptr;
-    cudaError_t e = cudaMalloc(&d_out, ob);
+    cudaError_t e = device_alloc(ctx, &d_out, ob);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "count scratch");
     const igxrt_status st = trace_common(ctx, scene, rays, prev_hit, count, mode, d_out, 0, stream,

@@ -119,7 +119,9 @@ inline size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // Idle bytes a context's pool keeps.
 constexpr uint64_t kPoolKeep = 1ull << 30;
 
-// Memory from the context's pool, ordered on `stream`; from cudaMalloc where
+// cudaMalloc, which gets the pool's idle memory too where it would fail.
+cudaError_t device_alloc(igxrt_context* ctx, void** ptr, size_t bytes);
+// Memory from the context's pool, ordered on `stream`; from device_alloc where
 // there is no pool or it cannot serve the size (`pooled` says which).
 cudaError_t pool_alloc(igxrt_context* ctx, void** ptr, size_t bytes, cudaStream_t stream, bool& pooled);
 

@@ -456,7 +456,8 @@ igxrt_status igxrt_scene_refit(igxrt_context* ctx, igxrt_scene* scene, const igx
 
     const uint32_t n = a.obj.count();
     if (n && !scene->refit_boxes) {  // once per scene, at its first refit
-        const cudaError_t e = cudaMalloc(&scene->refit_boxes, 2 * sizeof(float4) * (size_t)n);
+        const cudaError_t e =
+            device_alloc(ctx, reinterpret_cast<void**>(&scene->refit_boxes), 2 * sizeof(float4) * (size_t)n);
         if (e != cudaSuccess) {
             scene->refit_boxes = nullptr;
             return cuda_fail(ctx, e, "refit scratch allocation");

@@ -405,7 +405,7 @@ igxrt_status igxrt_server_create(igxrt_context* ctx, const igxrt_server_options*
     if (!guard.ok())
         return fail(ctx, IGXRT_ERROR_CUDA, "cannot select the context's device");
     s->opt.memory_cap_bytes = round256(s->opt.memory_cap_bytes);
-    cudaError_t e = cudaMalloc(&s->d_arena, s->opt.memory_cap_bytes);
+    cudaError_t e = device_alloc(ctx, reinterpret_cast<void**>(&s->d_arena), s->opt.memory_cap_bytes);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "server arena (memory_cap_bytes)");
     s->arena.reset(new Arena(s->opt.memory_cap_bytes));

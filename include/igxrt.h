@@ -303,6 +303,11 @@ igxrt_status igxrt_scene_create_from_bvh(igxrt_context* ctx, const igxrt_bvh* bv
  * max_leaf_size is used (0 = 4): a subtree of at most that many objects
  * becomes one leaf.  The work is ordered on `stream`; the call returns once
  * the scene is ready.
+ *
+ * Scratch and scene come from a memory pool of the context, which keeps up to
+ * 1 GiB of device memory for the next build (other allocators see it as taken)
+ * until the context and the last scene built from it are destroyed; the
+ * context's own allocations take it back before they fail.
  */
 igxrt_status igxrt_scene_create_gpu(igxrt_context* ctx, const igxrt_scene_desc* desc,
                                     const igxrt_build_options* opts, uint32_t flags, void* stream,
