@@ -8,8 +8,9 @@
 // carry their own item (node array, records, output, query mode): a warp can
 // finish rays of one scene while starting rays of the next, and the GPU stays
 // full across item boundaries instead of draining at the end of each launch.
-// Per ray the traversal is the plain kernel's (same visiting order, same
-// arithmetic, and the same tail work sharing once the queue is drained), so
+// Per ray the node visits and the arithmetic are the plain kernel's, with the
+// same tail work sharing once the queue is drained (leaves are taken lane by
+// lane, where the plain kernels over grid nodes deal them over the warp), so
 // results equal tracing each item alone.
 #include <algorithm>
 #include <cstring>

@@ -141,8 +141,8 @@ bool grid_usable(const uint32_t* words);
 // Launches over a scene with grid nodes use them in place of the two layouts
 // of exact boxes, whichever of the two the caller names: both find the same
 // hits, and the grid nodes were the faster at every size measured (a 1M
-// sphere's primaries 471 -> 440 us, 4M incoherent rays over 2M triangles
-// 3,003 -> 2,398 us).  BVH8 stays as named.
+// sphere's primaries 471 us over BVH2 and 388 so, 4M incoherent rays over 2M
+// triangles 3,003 and 2,160 us).  BVH8 stays as named.
 inline bool use_grid(const igxrt_scene& s, uint32_t layout) { return s.grid_ok && layout != IGXRT_LAYOUT_BVH8; }
 // A scene without nodes takes part in any launch.
 inline bool grid_or_empty(const igxrt_scene& s, uint32_t layout) {

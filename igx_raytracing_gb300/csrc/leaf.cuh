@@ -28,7 +28,7 @@ namespace igxrt {
 // Lanes waiting (at a leaf, or done) that end the node phase: 14, 20 and never
 // (the rule of phase_break alone) gave 388, 397 and 403 us on the sphere's
 // primaries, 2,166, 2,205 and 2,239 on the incoherent rays, 248, 248 and 252
-// on the shadow rays; 10 gave the shadow rays 262 where 14 gave 262.
+// on the shadow rays.
 constexpr uint32_t kLeafLanes = 14;
 
 // A warp's part of shared memory, after the block's stacks.

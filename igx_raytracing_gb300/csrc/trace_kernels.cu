@@ -4,9 +4,9 @@
 // CTAs stay resident, each warp repeatedly takes a packet of `packet` rays
 // from a global atomic work queue and its lanes trace them, so uneven ray
 // costs (a miss of the root box vs. a deep closest hit) balance across the
-// GPU without a tail of idle SMs.  Node and primitive records are read with
-// 128-bit read-only loads; hit records are written with streaming stores so
-// they do not displace BVH lines from L2.
+// GPU without a tail of idle SMs.  Nodes are read with 256-bit and primitive
+// records with 128-bit read-only loads; hit records are written with streaming
+// stores so they do not displace BVH lines from L2.
 #include <algorithm>
 #include <type_traits>
 
@@ -119,14 +119,17 @@ constexpr int trace_kernel_regs(int layout, bool any, bool mixed) {
 // Persistent traversal.  Every lane owns one ray at a time; a warp alternates
 // a node phase (each lane descends until it reaches a leaf or finishes, or
 // until few lanes still descend: node_phase) and a leaf phase (each lane at
-// a leaf tests it), so lanes at the same kind of work execute together.  Between phases, once `refill_lanes` lanes are idle the
-// warp hands them new rays: one atomicAdd on the global queue claims a
-// packet of `packet` ray indices for the warp, and idle lanes take the next
-// indices in lane order (ballot + popc).  Until the warp finds the queue
-// drained, and always in the instrumented (COUNT) kernels, each ray's
-// sequence of node and leaf visits is exactly the host traversal's
-// (oracle/trace_oracle.c); after that share_tail splits rays across lanes,
-// which visits the same subtrees in another order with the same result.
+// a leaf tests it, or the warp tests all of them: leaf.cuh), so lanes at the
+// same kind of work execute together.  Between phases, once `refill_lanes`
+// lanes are idle the warp hands them new rays: one atomicAdd on the global
+// queue claims a packet of `packet` ray indices for the warp, and idle lanes
+// take the next indices in lane order (ballot + popc).  Over the exact layouts
+// each ray's sequence of node and leaf visits is the host traversal's
+// (oracle/trace_oracle.c) until the warp finds the queue drained, and always in
+// the instrumented (COUNT) kernels; after that share_tail splits rays across
+// lanes, which visits the same subtrees in another order with the same result.
+// The grid nodes have no host traversal: their boxes are larger and a visit's
+// order differs among boxes behind the origin, with the same result again.
 // MIXED: scenes with spheres, cubes and planes (typed leaves, planes tested
 // when a ray starts, priority-coded best hit).  CAMERA: ray i is made in the
 // kernel, the camera's primary ray of pixel i in row-major order

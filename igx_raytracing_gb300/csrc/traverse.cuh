@@ -8,8 +8,9 @@
 //     to right, cross products in GLSL component order, f = 1/a correctly
 //     rounded (__frcp_rn), denormals kept (the library is built without
 //     -ftz);
-//   * the slab test uses explicit fmaf on both sides so the host and the GPU
-//     cull the same boxes and visit nodes in the same order;
+//   * over the exact layouts the slab test uses explicit fmaf on both sides so
+//     the host and the GPU cull the same boxes and visit nodes in the same order
+//     (the grid nodes' test is grid.cuh's, which no host traversal repeats);
 //   * a hit (t, prim) replaces the best one when t < best.t, or t == best.t
 //     and prim < best.prim: the linear loop's "first index reaching the
 //     smallest t" (trace.glsl:25-27 with the strict t >= hit.hitT rejection at

@@ -371,7 +371,8 @@ typedef struct igxrt_launch_params {
     uint32_t packet_size; /* rays a warp claims per queue fetch: a multiple of
                              8 up to 4096; 0 = 16 */
     uint32_t layout;      /* IGXRT_LAYOUT_*; BVH2 and BVH4 launches trace the engine's own quantized
-                             form of the BVH4 nodes instead where the scene has one (same hits) */
+                             form of the BVH4 nodes instead where the scene has one (same hits), but
+                             for igxrt_trace_gbuffer on mixed scenes or host images in place */
     uint32_t ctas_per_sm; /* persistent CTAs per SM, 0 = as many as fit */
     uint32_t refill_lanes;/* a warp refetches rays once this many of its lanes
                              are idle (1..32); 0 = 8 */
@@ -379,8 +380,10 @@ typedef struct igxrt_launch_params {
                              together, then test their leaves together; the
                              descent ends early once phase_break times the
                              lanes still descending is at most the number of
-                             lanes waiting (at a leaf, or done), and those
-                             lanes resume after the leaves.  1..31; 32 = no
+                             lanes waiting (at a leaf, or done), or, where
+                             triangle scenes are traced in the quantized form
+                             of `layout`, once 14 lanes wait; the others
+                             resume after the leaves.  1..31; 32 = no
                              early end (every lane reaches a leaf first);
                              0 = 2.  Results do not depend on it. */
     uint32_t reserved;
