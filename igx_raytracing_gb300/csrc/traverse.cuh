@@ -598,10 +598,10 @@ __device__ __forceinline__ void sphere_offset(const RayState& r, float cx, float
 }
 
 // The sphere's uv (the rest of primitive.glsl:189-204) from sphere_offset.
-// asin and atan give the correctly rounded binary32 value: evaluated in binary64 (CUDA's asin /
-// atan, a few binary64 ulp) and rounded once, which lands on the correctly
-// rounded float unless the binary64 value falls within its error of a
-// binary32 rounding midpoint.  The oracle evaluates them the same way, so u
+// asin and atan give the correctly rounded binary32 value: evaluated in
+// binary64 (CUDA's asin / atan, a few binary64 ulp) and rounded once, which
+// lands on the correctly rounded float unless the binary64 value falls within
+// its error of a binary32 rounding midpoint.  The oracle evaluates them the same way, so u
 // and v, which cancel towards 0 near the poles and the seam (lat * 1/pi +
 // 0.5), come out bit for bit instead of many float ulp apart.
 __device__ __forceinline__ void sphere_uv(float nx, float ny, float nz, float& u, float& v) {

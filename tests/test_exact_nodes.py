@@ -218,3 +218,11 @@ def test_ordinary_scenes_are_on_the_grid(ctx, leaf):
         scene = ctx.create_scene(tris, max_leaf_size=leaf)
         assert uses_grid(scene)
         scene.close()
+
+
+def test_detail_below_the_grid_steps_stays_exact(ctx):
+    from test_grid import _stadium
+
+    scene = ctx.create_scene(_stadium(8160))
+    assert not uses_grid(scene)
+    scene.close()
